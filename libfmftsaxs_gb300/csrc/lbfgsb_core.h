@@ -930,28 +930,71 @@ typedef struct {
 
 #define LB_X(o, c, i) ((o)->cr[((long)(c) * (o)->Q + (i)) * (o)->stride])
 
-LB_HD double lb_in(const lb_saxs *o, int i, double G, double c2)
+/* The model and its derivatives at one q: x[c] the six cross terms there */
+LB_HD double lb_in(const double *x, double G, double c2)
 {
-	return LB_X(o, 0, i) - G * LB_X(o, 1, i) + c2 * LB_X(o, 2, i) + G * G * LB_X(o, 3, i) - G * c2 * LB_X(o, 4, i) +
-	       c2 * c2 * LB_X(o, 5, i);
+	return x[0] - G * x[1] + c2 * x[2] + G * G * x[3] - G * c2 * x[4] + c2 * c2 * x[5];
+}
+LB_HD double lb_gder(double G, double c1, double mult, double q) { return G * (3.0 / c1 - 2.0 * c1 * mult * q * q); }
+LB_HD double lb_idc1(const double *x, double G, double Gd, double c2)
+{
+	return Gd * (-x[1] + 2.0 * G * x[3] - c2 * x[4]);
+}
+/* the reference's derivative before the first point has its own rounding */
+LB_HD double lb_idc1_first(const double *x, double G, double Gd, double c2)
+{
+	return -Gd * x[1] + 2.0 * G * Gd * x[3] - Gd * c2 * x[4];
+}
+LB_HD double lb_idc2(const double *x, double G, double c2) { return x[2] - G * x[4] + 2.0 * c2 * x[5]; }
+
+/* The terms that one q adds to the sums of sxs_best_scale
+ * (src/min_saxs.c:261-319): up = t[0], down = t[1]; a the bin's moments */
+LB_HD void lb_scale_terms(double in, double tan, double q, const double *a, double *t)
+{
+	double buf = in - tan * q;
+	t[0] = buf * a[1] + tan * a[2];
+	t[1] = buf * buf * a[3] + 2.0 * tan * buf * a[4] + tan * tan * a[5];
+}
+/* the terms of the gradient (t[0], t[1]) and of chi^2 (t[2]) at fixed scale
+ * k (src/min_saxs.c:3-105) */
+LB_HD void lb_grad_terms(double k, double q, const double *a, double in, double tan, double i1, double t1, double i2,
+                         double t2, double *t)
+{
+	t[0] = 2.0 * k * (-(i1 - t1 * q) * a[1] - t1 * a[2] +
+	                  k * ((in - tan * q) * (i1 - t1 * q) * a[3] + (in * t1 + i1 * tan - 2.0 * tan * t1 * q) * a[4] +
+	                       tan * t1 * a[5]));
+	t[1] = 2.0 * k * (-(i2 - t2 * q) * a[1] - t2 * a[2] +
+	                  k * ((in - tan * q) * (i2 - t2 * q) * a[3] + (in * t2 + i2 * tan - 2.0 * tan * t2 * q) * a[4] +
+	                       tan * t2 * a[5]));
+	double buf = in - tan * q;
+	t[2] = a[0] + k * (-2.0 * buf * a[1] - 2.0 * tan * a[2] +
+	                   k * (buf * buf * a[3] + 2.0 * buf * tan * a[4] + tan * tan * a[5]));
+}
+
+LB_HD void lb_load(const lb_saxs *o, int i, double *x)
+{
+	for (int c = 0; c < 6; c++) x[c] = LB_X(o, c, i);
 }
 
 /* sxs_best_scale (src/min_saxs.c:261-319) */
 LB_HD double lb_best_scale(const lb_saxs *o, double c1, double c2)
 {
-	const double *q = o->q, *a = o->a;
+	const double *q = o->q;
+	double x[6], t[2];
 	double corr = -o->mult * (c1 * c1 - 1.0);
 	double G = c1 * c1 * c1 * exp(corr * q[0] * q[0]);
-	double in_prev = lb_in(o, 0, G, c2);
+	lb_load(o, 0, x);
+	double in_prev = lb_in(x, G, c2);
 	double c1c = c1 * c1 * c1, q_prev = -1.0, up = 0.0, down = 0.0;
 	for (int i = 0; i < o->Q; i++) {
 		double qc = q[i];
 		G = c1c * exp(corr * qc * qc);
-		double in = lb_in(o, i, G, c2);
+		lb_load(o, i, x);
+		double in = lb_in(x, G, c2);
 		double tan = (in - in_prev) / (qc - q_prev);
-		double buf = in - tan * qc;
-		up += buf * a[i * 6 + 1] + tan * a[i * 6 + 2];
-		down += buf * buf * a[i * 6 + 3] + 2.0 * tan * buf * a[i * 6 + 4] + tan * tan * a[i * 6 + 5];
+		lb_scale_terms(in, tan, qc, o->a + i * 6, t);
+		up += t[0];
+		down += t[1];
 		in_prev = in;
 		q_prev = qc;
 	}
@@ -961,40 +1004,32 @@ LB_HD double lb_best_scale(const lb_saxs *o, double c1, double c2)
 /* gradient and chi^2 at fixed scale k (src/min_saxs.c:3-105) */
 LB_HD void lb_gradient(const lb_saxs *o, const double *x, double k, double *grad, double *score_val)
 {
-	const double *q = o->q, *a = o->a;
-	double c1 = x[0], c2 = x[1], mult = o->mult;
+	const double *q = o->q;
+	double c1 = x[0], c2 = x[1], mult = o->mult, cr[6], t[3];
 	double g0 = 0.0, g1 = 0.0;
 	double corr = -mult * (c1 * c1 - 1.0);
 	double G = c1 * c1 * c1 * exp(corr * q[0] * q[0]);
-	double G_der = G * (3.0 / c1 - 2.0 * c1 * mult * q[0] * q[0]);
-	double in_prev = lb_in(o, 0, G, c2);
-	double idc1_prev = -G_der * LB_X(o, 1, 0) + 2.0 * G * G_der * LB_X(o, 3, 0) - G_der * c2 * LB_X(o, 4, 0);
-	double idc2_prev = LB_X(o, 2, 0) - G * LB_X(o, 4, 0) + 2.0 * c2 * LB_X(o, 5, 0);
+	double Gd = lb_gder(G, c1, mult, q[0]);
+	lb_load(o, 0, cr);
+	double in_prev = lb_in(cr, G, c2);
+	double i1_prev = lb_idc1_first(cr, G, Gd, c2);
+	double i2_prev = lb_idc2(cr, G, c2);
 	double q_prev = -1.0, score = 0.0, c1c = c1 * c1 * c1;
 	for (int i = 0; i < o->Q; i++) {
 		double qc = q[i];
 		G = c1c * exp(corr * qc * qc);
-		G_der = G * (3.0 / c1 - 2.0 * c1 * mult * qc * qc);
-		double in = lb_in(o, i, G, c2);
-		double idc1 = G_der * (-LB_X(o, 1, i) + 2.0 * G * LB_X(o, 3, i) - c2 * LB_X(o, 4, i));
-		double idc2 = LB_X(o, 2, i) - G * LB_X(o, 4, i) + 2.0 * c2 * LB_X(o, 5, i);
+		Gd = lb_gder(G, c1, mult, qc);
+		lb_load(o, i, cr);
+		double in = lb_in(cr, G, c2), i1 = lb_idc1(cr, G, Gd, c2), i2 = lb_idc2(cr, G, c2);
 		double buf = 1.0 / (qc - q_prev);
-		double tan = (in - in_prev) * buf;
-		double t1 = (idc1 - idc1_prev) * buf;
-		double t2 = (idc2 - idc2_prev) * buf;
-		const double *ai = a + i * 6;
-		g0 += 2.0 * k * (-(idc1 - t1 * qc) * ai[1] - t1 * ai[2] +
-		                 k * ((in - tan * qc) * (idc1 - t1 * qc) * ai[3] +
-		                      (in * t1 + idc1 * tan - 2.0 * tan * t1 * qc) * ai[4] + tan * t1 * ai[5]));
-		g1 += 2.0 * k * (-(idc2 - t2 * qc) * ai[1] - t2 * ai[2] +
-		                 k * ((in - tan * qc) * (idc2 - t2 * qc) * ai[3] +
-		                      (in * t2 + idc2 * tan - 2.0 * tan * t2 * qc) * ai[4] + tan * t2 * ai[5]));
-		buf = in - tan * qc;
-		score += ai[0] + k * (-2.0 * buf * ai[1] - 2.0 * tan * ai[2] +
-		                      k * (buf * buf * ai[3] + 2.0 * buf * tan * ai[4] + tan * tan * ai[5]));
+		lb_grad_terms(k, qc, o->a + i * 6, in, (in - in_prev) * buf, i1, (i1 - i1_prev) * buf, i2, (i2 - i2_prev) * buf,
+		              t);
+		g0 += t[0];
+		g1 += t[1];
+		score += t[2];
 		in_prev = in;
-		idc1_prev = idc1;
-		idc2_prev = idc2;
+		i1_prev = i1;
+		i2_prev = i2;
 		q_prev = qc;
 	}
 	grad[0] = g0;
@@ -1021,14 +1056,15 @@ LB_HD void lb_reset_memory(lb_state *s)
 }
 
 /* The fit of src/min_saxs.c:196-259: x0 = (1, 0), bounds [0.96, 1.04] x
- * [-2, 4], m = 3, factr = 1e7, pgtol = 1e-5.  Returns the number of
- * objective evaluations; chi = sqrt(f), scale = best scale at the result.
- * max_eval bounds the work per pose (the reference has no bound; the
- * algorithm stops long before it in practice). */
-LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, double *scale, int max_eval)
+ * [-2, 4], m = 3, factr = 1e7, pgtol = 1e-5, in reverse communication:
+ * lb_fit_begin sets s->x; then each lb_fit_advance takes the f and g of
+ * s->x (first != 0: of the starting point) and either moves s->x to the next
+ * point to evaluate (returns 1) or ends with the result in s->x, s->f
+ * (returns 0).  nevals = evaluations so far; max_eval bounds the work per
+ * pose (the reference has no bound; the algorithm stops long before it in
+ * practice). */
+LB_HD void lb_fit_begin(lb_state *s)
 {
-	lb_state st;
-	lb_state *s = &st;
 	const int n = LB_N;
 	s->x[0] = 1.0; s->x[1] = 0.0;
 	s->l[0] = 0.96; s->l[1] = -2.00;
@@ -1070,18 +1106,23 @@ LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, dou
 			V1(s->iwhere, i) = (V1(s->nbd, i) == 2 && V1(s->u, i) - V1(s->l, i) <= 0.0) ? 3 : 0;
 		}
 	}
-	int nevals = 0;
-	double sc = 1.0;
-	lb_eval(s, o, &sc);
-	nevals++;
+}
+
+LB_HD int lb_fit_advance(lb_state *s, int first, int nevals, int max_eval)
+{
+	const int n = LB_N;
+	const double pgtol = 1e-5;
+	int wrk, info, new_x, finfo;
+	double rr, dr, ddum;
+	if (!first) goto evaluated;
 	s->nfgv = 1;
 	lb_projgr(s, &s->sbgnrm);
-	const double pgtol = 1e-5;
-	if (s->sbgnrm <= pgtol) goto done;
+	if (s->sbgnrm <= pgtol) return 0;
 	for (;;) {
 		/* L222 */
 		s->iword = -1;
-		int wrk = 0, info = 0;
+		wrk = 0;
+		info = 0;
 		if (!s->cnstnd && s->col > 0) {
 			for (int i = 0; i < n; i++) s->z[i] = s->x[i];
 			wrk = s->updatd;
@@ -1139,8 +1180,8 @@ LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, dou
 		s->fold = s->f;
 		s->ifun = 0;
 		s->iback = 0;
-		int task = LS_START;
-		int new_x = 0;
+		s->ls_task = LS_START;
+		new_x = 0;
 		for (;;) {
 			s->gd = lb_dot(n, s->g, s->d);
 			if (s->ifun == 0) {
@@ -1150,9 +1191,9 @@ LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, dou
 					break;
 				}
 			}
-			lb_dcsrch(s, s->f, s->gd, &s->stp, s->stpmx, &task);
+			lb_dcsrch(s, s->f, s->gd, &s->stp, s->stpmx, &s->ls_task);
 			s->xstep = s->stp * s->dnorm;
-			if (task != LS_WARN && task != LS_CONV) {
+			if (s->ls_task != LS_WARN && s->ls_task != LS_CONV) {
 				++s->ifun;
 				++s->nfgv;
 				s->iback = s->ifun - 1;
@@ -1162,9 +1203,10 @@ LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, dou
 					for (int i = 0; i < n; i++) s->x[i] = s->stp * s->d[i] + s->t[i];
 				}
 				if (s->iback >= 20) break; /* checked before the evaluation */
-				if (nevals >= max_eval) goto done;
-				lb_eval(s, o, &sc);
-				nevals++;
+				if (nevals >= max_eval) return 0;
+				return 1;
+evaluated:
+				new_x = 0;
 			} else {
 				new_x = 1;
 				break;
@@ -1175,7 +1217,7 @@ LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, dou
 			for (int i = 0; i < n; i++) { s->x[i] = s->t[i]; s->g[i] = s->r[i]; }
 			s->f = s->fold;
 			if (s->col == 0) {
-				goto done; /* abnormal termination */
+				return 0; /* abnormal termination */
 			}
 			lb_reset_memory(s);
 			continue;
@@ -1183,13 +1225,11 @@ LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, dou
 		++s->iter;
 		lb_projgr(s, &s->sbgnrm);
 		/* L777: termination tests */
-		if (s->sbgnrm <= pgtol) goto done;
-		{
-			double ddum = lb_max(lb_max(lb_abs(s->fold), lb_abs(s->f)), 1.0);
-			if (s->fold - s->f <= s->tol * ddum) goto done;
-		}
+		if (s->sbgnrm <= pgtol) return 0;
+		ddum = lb_max(lb_max(lb_abs(s->fold), lb_abs(s->f)), 1.0);
+		if (s->fold - s->f <= s->tol * ddum) return 0;
 		for (int i = 0; i < n; i++) s->r[i] = s->g[i] - s->r[i];
-		double rr = lb_dot(n, s->r, s->r), dr, ddum;
+		rr = lb_dot(n, s->r, s->r);
 		if (s->stp == 1.0) {
 			dr = s->gd - s->gdold;
 			ddum = -s->gdold;
@@ -1205,15 +1245,28 @@ LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, dou
 		s->updatd = 1;
 		++s->iupdat;
 		lb_matupd(s, rr, dr);
-		int finfo = 0;
+		finfo = 0;
 		lb_formt(s, &finfo);
 		if (finfo != 0) lb_reset_memory(s);
 	}
-done:
-	*chi = sqrt(s->f);
-	*c1 = s->x[0];
-	*c2 = s->x[1];
-	*scale = lb_best_scale(o, s->x[0], s->x[1]);
+}
+
+/* One pose alone.  Returns the number of objective evaluations; chi =
+ * sqrt(f), scale = best scale at the result. */
+LB_HD int lb_saxs_fit(const lb_saxs *o, double *chi, double *c1, double *c2, double *scale, int max_eval)
+{
+	lb_state st;
+	int nevals = 0;
+	double sc = 1.0;
+	lb_fit_begin(&st);
+	do {
+		lb_eval(&st, o, &sc);
+		nevals++;
+	} while (lb_fit_advance(&st, nevals == 1, nevals, max_eval));
+	*chi = sqrt(st.f);
+	*c1 = st.x[0];
+	*c2 = st.x[1];
+	*scale = lb_best_scale(o, st.x[0], st.x[1]);
 	return nevals;
 }
 

@@ -241,9 +241,8 @@ struct sxsg_plan {
 	size_t r_budget;
 	/* outputs */
 	/* cross terms [npose][6][Q]: double on the FP64 path, double-float
-	 * pairs {hi, lo} (same size) on the mixed path; d_scaled is the
-	 * L-BFGS-B fit's rescaled, transposed copy, allocated on its first use */
-	double *d_cross, *d_chi, *d_c1, *d_c2, *d_grid, *d_scaled, *d_scale;
+	 * pairs {hi, lo} (same size) on the mixed path */
+	double *d_cross, *d_chi, *d_c1, *d_c2, *d_grid, *d_scale;
 	int32_t *d_cell;
 	int *d_iters;
 	size_t out_cap;
@@ -291,7 +290,7 @@ void sxsg_plan_destroy(sxsg_plan *p)
 		pfree(p, p->d_U);
 	}
 	pfree(p, p->d_cross); pfree(p, p->d_chi); pfree(p, p->d_c1); pfree(p, p->d_c2); pfree(p, p->d_grid);
-	pfree(p, p->d_scaled); pfree(p, p->d_scale); pfree(p, p->d_cell); pfree(p, p->d_iters);
+	pfree(p, p->d_scale); pfree(p, p->d_cell); pfree(p, p->d_iters);
 	for (int i = 0; i < 6; i++) if (p->ev[i]) cudaEventDestroy(p->ev[i]);
 	if (p->s2) cudaStreamDestroy(p->s2);
 	for (int i = 0; i < p->ncev; i++) cudaEventDestroy(p->cev[i]);
@@ -661,9 +660,9 @@ int sxsg_plan_set_poses(sxsg_plan *p, const int64_t *index, int64_t n, int skip)
 	size_t need = (size_t)nn;
 	if ((rc = grow(p, (void **)&p->d_cross, &p->out_cap, need * 6 * p->Q, sizeof(double)))) return rc;
 	/* out_cap tracks d_cross in doubles; the per-pose vectors follow it */
-	pfree(p, p->d_chi); pfree(p, p->d_c1); pfree(p, p->d_c2); pfree(p, p->d_cell); pfree(p, p->d_scaled);
+	pfree(p, p->d_chi); pfree(p, p->d_c1); pfree(p, p->d_c2); pfree(p, p->d_cell);
 	pfree(p, p->d_scale); pfree(p, p->d_iters); pfree(p, p->d_grid);
-	p->d_chi = p->d_c1 = p->d_c2 = p->d_scaled = p->d_scale = p->d_grid = NULL;
+	p->d_chi = p->d_c1 = p->d_c2 = p->d_scale = p->d_grid = NULL;
 	p->d_cell = NULL; p->d_iters = NULL;
 	e = cudaMallocAsync((void **)&p->d_chi, sizeof(double) * nn, p->s);
 	if (!e) e = cudaMallocAsync((void **)&p->d_c1, sizeof(double) * nn, p->s);
@@ -828,8 +827,7 @@ void sxs_plan_mark_run(sxsg_plan *p, int fit_mode, const float *ms)
 
 /* Host work before a run's launches: the twiddles (host copy kept with the
  * plan, so the upload needs no wait), the tensor-core scratch, the
- * translated table's chunking, its buffer and the timing events, the
- * L-BFGS-B workspace.  After it, sxs_plan_enqueue issues only stream work
+ * translated table's chunking, its buffer and the timing events.  After it, sxs_plan_enqueue issues only stream work
  * that a CUDA graph can capture. */
 int sxs_plan_prepare(sxsg_plan *p, int fit_mode)
 {
@@ -897,8 +895,6 @@ int sxs_plan_prepare(sxsg_plan *p, int fit_mode)
 	p->h_chunk[nch] = p->nslice;
 	if (nch > INT32_MAX / 3) return sxs_fail(-2, "sxsg_plan_run: too many chunks");
 	if ((rc = plan_events(p, (int)(3 * nch)))) return rc;
-	if (fit_mode == SXSG_FIT_LBFGSB && !p->d_scaled && p->npose > 0)
-		SXS_CU(cudaMallocAsync((void **)&p->d_scaled, sizeof(double) * (size_t)p->npose * 6 * p->Q, s));
 	p->run_nch = nch;
 	p->last_chunks = (int)(nch < INT32_MAX ? nch : INT32_MAX);
 	return 0;
@@ -948,9 +944,9 @@ int sxs_plan_enqueue(sxsg_plan *p, int fit_mode, int timed)
 		SXS_K(plan_fit_grid(p, n, p->d_chi, p->d_c1, p->d_c2, p->d_cell, NULL, s));
 		sxs_count_launches(n > 0 ? 1 : 0);
 	} else if (fit_mode == SXSG_FIT_LBFGSB) {
-		SXS_K(sxs_fit_lbfgsb_launch(p->d_cross, p->fp32, p->d_scaled, n, Q, p->d_q, p->d_a, p->mult, p->peak, 1, p->d_chi,
+		SXS_K(sxs_fit_lbfgsb_launch(p->d_cross, p->fp32, n, Q, p->d_q, p->d_a, p->mult, p->peak, 1, p->d_chi,
 		                            p->d_c1, p->d_c2, p->d_scale, p->d_iters, s));
-		sxs_count_launches(n > 0 ? 2 : 0);
+		sxs_count_launches(n > 0 ? 1 : 0);
 		if (n > 0) SXS_CU(cudaMemsetAsync(p->d_cell, 0xff, sizeof(int32_t) * n, s));
 	}
 	p->last_fit = fit_mode;
@@ -1121,7 +1117,7 @@ size_t sxs_plan_table_bytes(int L, int Q, int precision)
 
 /* Device bytes of a plan besides its rotation tables and translated-table
  * chunk: molecules, per-z tables for nzt touched z, pose lists and outputs. */
-size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int precision, int fit_mode)
+size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int precision)
 {
 	size_t K = L + 1, N = 2 * L + 1, NT = (Q + SXS_QT - 1) / SXS_QT, K2 = K * K;
 	size_t celem = precision == SXSG_MIXED ? 8 : 16;
@@ -1130,7 +1126,6 @@ size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int pre
 	b += (size_t)nzt * Q * N * 8;                                /* Bessel */
 	b += NT * nzt * K * K * K * SXS_QT * (precision == SXSG_MIXED ? 12 : 8); /* tau */
 	b += (size_t)npose * (sizeof(sxsk_pose) + 6 * Q * 8 + 40);   /* poses, cross, outputs */
-	if (fit_mode == SXSG_FIT_LBFGSB) b += (size_t)npose * 6 * Q * 8; /* its rescaled copy */
 	b += (size_t)n1 * Q * 16 + (size_t)64 * Q + (1 << 20);
 	return b;
 }

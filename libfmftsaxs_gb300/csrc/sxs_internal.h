@@ -72,7 +72,7 @@ int sxs_plan_create_on(sxsg_plan **out, const double *A, const double *B, const 
                        const double *c2g, int n2, int precision, cudaStream_t stream, int ext_tables);
 void sxs_plan_set_tables(sxsg_plan *p, void *P, int P_valid, void *U, int U_valid);
 size_t sxs_plan_table_bytes(int L, int Q, int precision);
-size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int precision, int fit_mode);
+size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int precision);
 size_t sxs_plan_combo_bytes(int L, int Q, int precision);
 
 /* What a batch of plans (sxs_batch.c) reads of one plan: its sizes, the
@@ -116,13 +116,12 @@ int sxs_pack_first_fit(const size_t *bytes, size_t n, size_t cap, int *phase, si
 /* per-q constants of the grid fit: fc[Q][5] */
 void sxs_fit_constants(const double *q, const double *a, int Q, double *fc);
 
-/* device L-BFGS-B over (c1, c2) for a batch of poses: cross [n][6][Q]
- * (rescaled here by peak when rescale != 0), ct a workspace of n*6*Q
- * doubles; two kernel launches */
-/* cross: double, or double-float pairs {hi, lo} when cross_df (the mixed
- * path's per-pose terms) */
-int sxs_fit_lbfgsb_launch(const void *cross, int cross_df, double *ct, int npose, int Q, const double *q,
-                          const double *a, double mult, double peak, int rescale, double *chi, double *c1, double *c2,
-                          double *scale, int *nevals, cudaStream_t s);
+/* device L-BFGS-B over (c1, c2) for a batch of poses: cross [n][6][Q],
+ * rescaled by peak in the kernel when rescale != 0; double, or double-float
+ * pairs {hi, lo} when cross_df (the mixed path's per-pose terms); one kernel
+ * launch */
+int sxs_fit_lbfgsb_launch(const void *cross, int cross_df, int npose, int Q, const double *q, const double *a,
+                          double mult, double peak, int rescale, double *chi, double *c1, double *c2, double *scale,
+                          int *nevals, cudaStream_t s);
 
 #endif
