@@ -100,6 +100,26 @@ size_t sxsk_rotate_tc_scratch(int L);
  * did not finish in either bounded wait: output invalid, its tensor memory
  * was not freed and the context must be considered unusable). */
 
+/* The plain path's contractions in fixed point (kernels_fixed.cu), L <=
+ * SXSK_FIX_LMAX: tables of the FP64 layouts and sizes whose complex entries
+ * are limbs {re h, re l, im h, im l} (int4), scaled per molecule and q.
+ * molecule: sc[2][Qp] (Qp = Q rounded up to 8) = {2^(28 - e), 2^e} of the
+ * flat coefficients, spf [3][K2][Q] their limbs (conjugated when conj);
+ * two launches.  dtab: limbs of a Wigner-d table.  tau: in place, the FP64
+ * matrices to limbs of tau / 2^nu, nu2[nz][Qp] = 2^nu a bound of their norm;
+ * two launches. */
+#define SXSK_FIX_LMAX 31
+int sxsk_fix_molecule(const double *flat, int Q, int L, int conj, double *sc, void *spf, cudaStream_t s);
+int sxsk_fix_dtab(const double *d, int2 *x, long n, cudaStream_t s);
+int sxsk_fix_tau(const double *bes, double *tau, int nz, int Q, int L, double *nu2, cudaStream_t s);
+int sxsk_fix_rotate(const void *spf, const int2 *dtab, const double2 *tw, int Q, int L, void *out, cudaStream_t s);
+/* as sxsk_translate and sxsk_pose_cross; combo_zbg = the chunk's combos */
+int sxsk_fix_translate(const void *U, const void *tau, const int32_t *combo_zbg, const int32_t *slices, int nslice,
+                       int cbase, int ncombo, int nzt, int Q, int L, void *R, cudaStream_t s);
+int sxsk_fix_cross(const sxsk_pose *poses, int npose, int combo_base, int ncombo, const int32_t *combo_zbg,
+                   const void *P, const void *R, const double2 *tw, const double *scA, const double *scB,
+                   const double *nu2, const double *cst, int Q, int L, double *cross, cudaStream_t s);
+
 /* Pose list on the device (src/index.c:3-29 packing, most significant
  * first: z slot, beta1, beta2, alpha2, gamma1, gamma2).  decode: one thread
  * per pose writes the decoded pose and its combo key (zi nb + b2) N + g2,

@@ -212,6 +212,10 @@ struct sxsg_plan {
 	float *d_amat;              /* twiddle operand of the tensor-core rotation */
 	int *d_tcstat;              /* its status word (kernels.h, sxsk_rotate_tc) */
 	int P_valid, U_valid;       /* caller tables already hold this run's rows */
+	int run_fixed;              /* the prepared run contracts in fixed point (sxs_plan_table_form) */
+	void *d_Ax, *d_Bx;          /* fixed point: limbs of the coefficients, their scales, and per z the */
+	double *d_scA, *d_scB;      /* matrices' scales (kernels.h), made by the first such run */
+	double *d_nu2;
 	int tw_variant; /* -1 none, 0 simple_ft, 1 exact */
 	double *h_tw;               /* host copy of the twiddles (lives with the plan) */
 	int64_t run_nch;            /* chunks of the prepared run */
@@ -270,8 +274,9 @@ static void plan_free_poses(sxsg_plan *p)
 	pfree(p, p->d_slices);
 	p->h_slices = NULL; p->d_slices = NULL; p->nslice = 0;
 	pfree(p, p->d_poses); pfree(p, p->d_combo); pfree(p, p->d_zt); pfree(p, p->d_bes); pfree(p, p->d_tau);
-	pfree(p, p->d_tauf); pfree(p, p->d_cstart);
+	pfree(p, p->d_tauf); pfree(p, p->d_cstart); pfree(p, p->d_nu2);
 	p->d_cstart = NULL;
+	p->d_nu2 = NULL;
 	p->h_combo = NULL; p->h_cstart = NULL; p->h_zt = NULL;
 	p->d_poses = NULL; p->d_combo = NULL; p->d_zt = NULL; p->d_bes = NULL; p->d_tau = NULL; p->d_tauf = NULL;
 }
@@ -285,6 +290,7 @@ void sxsg_plan_destroy(sxsg_plan *p)
 	pfree(p, p->d_A); pfree(p, p->d_B); pfree(p, p->d_q); pfree(p, p->d_fc); pfree(p, p->d_a); pfree(p, p->d_gtab); pfree(p, p->d_gdf);
 	pfree(p, p->d_c1g); pfree(p, p->d_c2g); pfree(p, p->d_cst); pfree(p, p->d_cstf); pfree(p, p->d_At); pfree(p, p->d_Bt);
 	pfree(p, p->d_tw); pfree(p, p->d_R); pfree(p, p->d_amat); pfree(p, p->d_tcstat); pfree(p, p->d_part);
+	pfree(p, p->d_Ax); pfree(p, p->d_Bx); pfree(p, p->d_scA); pfree(p, p->d_scB);
 	if (!p->ext_tables) {
 		pfree(p, p->d_P);
 		pfree(p, p->d_U);
@@ -675,14 +681,18 @@ int sxsg_plan_set_poses(sxsg_plan *p, const int64_t *index, int64_t n, int skip)
 	return 0;
 }
 
-/* per-z tables: Bessel values and translation matrices (FP64), with their
- * float copy on the mixed path */
+/* per-z tables: Bessel values and translation matrices (FP64), in limbs for
+ * a fixed-point run, with their float copy on the mixed path */
 static int plan_ztables(sxsg_plan *p, cudaStream_t s)
 {
 	int L = p->L, Q = p->Q;
 	SXS_K(sxsk_bessel_z(p->d_zt, p->nzt, p->d_q, Q, L, p->d_bes, s));
 	SXS_K(sxsk_tmatrix(p->d_bes, p->lt->d_dsymb, p->nzt, Q, L, p->lt->d_ll1, p->lt->nll1, p->d_tau, s));
 	sxs_count_launches(2);
+	if (p->run_fixed) {
+		SXS_K(sxsk_fix_tau(p->d_bes, p->d_tau, p->nzt, Q, L, p->d_nu2, s));
+		sxs_count_launches(2);
+	}
 	if (p->fp32) {
 		SXS_K(sxsk_to_float(p->d_tau, p->d_tauf, (long)p->NT * p->nzt * p->K * p->K * p->K * SXS_QT, s));
 		sxs_count_launches(1);
@@ -726,12 +736,14 @@ static int plan_rotations(sxsg_plan *p)
 		int tc = p->fp32 && p->rot_engine == SXSG_ROT_TC && 2 * N <= 128;
 		if (tc) SXS_CU(cudaMemsetAsync(p->d_tcstat, 0, sizeof(int), s));
 		if (!p->ext_tables || !p->P_valid) {
-			if (tc) SXS_K(sxsk_rotate_tc(p->d_At, p->lt->d_dtabf, p->d_tw, Q, L, 0, p->d_P, p->d_amat, p->d_tcstat, s));
+			if (p->run_fixed) SXS_K(sxsk_fix_rotate(p->d_Ax, p->lt->d_dtabx, p->d_tw, Q, L, p->d_P, s));
+			else if (tc) SXS_K(sxsk_rotate_tc(p->d_At, p->lt->d_dtabf, p->d_tw, Q, L, 0, p->d_P, p->d_amat, p->d_tcstat, s));
 			else SXS_K(sxsk_rotate(p->d_At, dtab, p->d_tw, Q, L, 0, p->d_P, p->fp32, p->rot_gamma, s));
 			sxs_count_launches(tc ? 2 : 1);
 		}
 		if (!p->ext_tables || !p->U_valid) {
-			if (tc) SXS_K(sxsk_rotate_tc(p->d_Bt, p->lt->d_dtabf, p->d_tw, Q, L, 1, p->d_U, p->d_amat, p->d_tcstat, s));
+			if (p->run_fixed) SXS_K(sxsk_fix_rotate(p->d_Bx, p->lt->d_dtabx, p->d_tw, Q, L, p->d_U, s));
+			else if (tc) SXS_K(sxsk_rotate_tc(p->d_Bt, p->lt->d_dtabf, p->d_tw, Q, L, 1, p->d_U, p->d_amat, p->d_tcstat, s));
 			else SXS_K(sxsk_rotate(p->d_Bt, dtab, p->d_tw, Q, L, 1, p->d_U, p->fp32, p->rot_gamma, s));
 			sxs_count_launches(tc ? 2 : 1);
 		}
@@ -825,6 +837,36 @@ void sxs_plan_mark_run(sxsg_plan *p, int fit_mode, const float *ms)
 	for (int i = 0; i < 5; i++) p->ms[i] = ms ? ms[i] : 0.0;
 }
 
+/* The contraction tables of a run.  On the plain path the fixed-point kernels
+ * (kernels_fixed.cu) take a quarter of the FP64 ones' time (L = 20, Q = 101,
+ * 70,000 poses: tables 4.0 against 17.0 ms, translation 16.0 / 59.2, poses
+ * 19.0 / 87.5) and are as close to the exact sums; they hold a column in
+ * registers up to L = 31.  The L-BFGS-B fit keeps the FP64 kernels: its stopping point
+ * moves by up to 1e-6 in (c1, c2) when the last bits of its input change. */
+int sxs_plan_table_form(int L, int precision, int fit_mode)
+{
+	if (precision != SXSG_FP64) return SXS_TABLES_FP32;
+	return L <= SXSK_FIX_LMAX && fit_mode != SXSG_FIT_LBFGSB ? SXS_TABLES_FIXED : SXS_TABLES_FP64;
+}
+
+/* what a fixed-point run reads beside the FP64 inputs: made once per plan
+ * (the coefficients' limbs) and per pose list (room for the scales) */
+static int plan_fixed_inputs(sxsg_plan *p)
+{
+	size_t Qp = (size_t)p->NT * SXS_QT, n = (size_t)3 * p->K2 * p->Q;
+	cudaStream_t s = p->s;
+	if (!p->d_nu2 && p->nzt > 0) SXS_CU(cudaMallocAsync((void **)&p->d_nu2, sizeof(double) * Qp * p->nzt, s));
+	if (p->d_Bx) return 0;
+	if (!p->d_scA) SXS_CU(cudaMallocAsync((void **)&p->d_scA, sizeof(double) * 2 * Qp, s));
+	if (!p->d_scB) SXS_CU(cudaMallocAsync((void **)&p->d_scB, sizeof(double) * 2 * Qp, s));
+	if (!p->d_Ax) SXS_CU(cudaMallocAsync(&p->d_Ax, sizeof(int4) * n, s));
+	SXS_K(sxsk_fix_molecule(p->d_A, p->Q, p->L, 0, p->d_scA, p->d_Ax, s));
+	SXS_CU(cudaMallocAsync(&p->d_Bx, sizeof(int4) * n, s));
+	SXS_K(sxsk_fix_molecule(p->d_B, p->Q, p->L, 1, p->d_scB, p->d_Bx, s));
+	sxs_count_launches(4);
+	return 0;
+}
+
 /* Host work before a run's launches: the twiddles (host copy kept with the
  * plan, so the upload needs no wait), the tensor-core scratch, the
  * translated table's chunking, its buffer and the timing events.  After it, sxs_plan_enqueue issues only stream work
@@ -851,6 +893,8 @@ int sxs_plan_prepare(sxsg_plan *p, int fit_mode)
 		SXS_CU(cudaMallocAsync((void **)&p->d_amat, sizeof(float) * sxsk_rotate_tc_scratch(p->L), s));
 	if (tc && !p->d_tcstat) SXS_CU(cudaMallocAsync((void **)&p->d_tcstat, sizeof(int), s));
 	p->run_fused = sxs_plan_uses_fused(p);
+	p->run_fixed = sxs_plan_table_form(p->L, p->precision, fit_mode) == SXS_TABLES_FIXED;
+	if (p->run_fixed && (rc = plan_fixed_inputs(p))) return rc;
 	free(p->h_chunk);
 	p->h_chunk = malloc(sizeof(int64_t) * (size_t)(p->nslice + 1));
 	if (!p->h_chunk) return sxs_fail(-5, "out of host memory");
@@ -927,6 +971,12 @@ int sxs_plan_enqueue(sxsg_plan *p, int fit_mode, int timed)
 			                           p->d_tw, p->d_part, s));
 			if (timed) SXS_CU(cudaEventRecord(e[1], s));
 			SXS_K(sxsk_fused_reduce(p->d_poses + p0, (int)(p1 - p0), p->d_part, Q, L, p->d_cstf, p->d_cross, s));
+		} else if (p->run_fixed) {
+			SXS_K(sxsk_fix_translate(p->d_U, tau, p->d_combo + 3 * c0, p->d_slices + 2 * s0, (int)(s1 - s0), (int)c0,
+			                         (int)(c1 - c0), p->nzt, Q, L, p->d_R, s));
+			if (timed) SXS_CU(cudaEventRecord(e[1], s));
+			SXS_K(sxsk_fix_cross(p->d_poses + p0, (int)(p1 - p0), (int)c0, (int)(c1 - c0), p->d_combo + 3 * c0, p->d_P,
+			                     p->d_R, p->d_tw, p->d_scA, p->d_scB, p->d_nu2, p->d_cst, Q, L, p->d_cross, s));
 		} else {
 			SXS_K(sxsk_translate(p->d_U, tau, p->d_combo + 3 * c0, p->d_slices + 2 * s0, (int)(s1 - s0), (int)c0,
 			                     (int)(c1 - c0), p->nzt, Q, L, p->d_R, p->fp32, p->tr_slices, s));
@@ -1126,6 +1176,7 @@ size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int pre
 	b += (size_t)nzt * Q * N * 8;                                /* Bessel */
 	b += NT * nzt * K * K * K * SXS_QT * (precision == SXSG_MIXED ? 12 : 8); /* tau */
 	b += (size_t)npose * (sizeof(sxsk_pose) + 6 * Q * 8 + 40);   /* poses, cross, outputs */
+	if (precision == SXSG_FP64) b += spf * 16 * 2 + (size_t)nzt * NT * SXS_QT * 8;   /* fixed-point inputs */
 	b += (size_t)n1 * Q * 16 + (size_t)64 * Q + (1 << 20);
 	return b;
 }

@@ -58,6 +58,7 @@ typedef struct {
 	int L;
 	double *d_dtab;   /* [K][K][N][N] */
 	float *d_dtabf;   /* the same in float (mixed-path rotation) */
+	int2 *d_dtabx;    /* the same in limbs (fixed-point rotation; NULL above its L) */
 	double *d_dsymb;  /* [K2][K][N] */
 	double *d_ynorm;  /* [K][N] */
 	int2 *d_ll1;      /* (l, l1 >= l) pairs */
@@ -70,6 +71,10 @@ int sxs_ltables_get(int L, const sxs_ltables **out);
 int sxs_plan_create_on(sxsg_plan **out, const double *A, const double *B, const double *q, int Q, const double *z,
                        int nz, int L, const double *a, double mult, double peak, const double *c1g, int n1,
                        const double *c2g, int n2, int precision, cudaStream_t stream, int ext_tables);
+/* form of the contraction tables of a run (rotation tables of one form are
+ * not readable by another) */
+enum { SXS_TABLES_FP64 = 0, SXS_TABLES_FP32 = 1, SXS_TABLES_FIXED = 2 };
+int sxs_plan_table_form(int L, int precision, int fit_mode);
 void sxs_plan_set_tables(sxsg_plan *p, void *P, int P_valid, void *U, int U_valid);
 size_t sxs_plan_table_bytes(int L, int Q, int precision);
 size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int precision);

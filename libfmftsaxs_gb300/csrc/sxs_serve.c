@@ -122,7 +122,7 @@ static uint64_t table_key(uint64_t mol, int role, const sxs_job *j, const double
 	if (!mol) return 0;
 	int K = j->L + 1;
 	uint64_t h = 1469598103934665603ull;
-	int v[5] = {role, j->L, j->Q, j->skip == 1, j->precision};
+	int v[5] = {role, j->L, j->Q, j->skip == 1, sxs_plan_table_form(j->L, j->precision, j->fit_mode)};
 	uint64_t d = digest(coef, (size_t)3 * j->Q * K * K * 2);
 	h = fnv(h, &mol, sizeof(mol));
 	h = fnv(h, &d, sizeof(d));

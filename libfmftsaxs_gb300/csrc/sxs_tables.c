@@ -310,10 +310,17 @@ int sxs_ltables_get(int L, const sxs_ltables **out)
 	cudaError_t e = cudaSuccess;
 	if (e == cudaSuccess) e = cudaMalloc((void **)&t->d_dtab, sizeof(double) * dsz * K);
 	if (e == cudaSuccess) e = cudaMalloc((void **)&t->d_dtabf, sizeof(float) * dsz * K);
+	if (e == cudaSuccess && L <= SXSK_FIX_LMAX) e = cudaMalloc((void **)&t->d_dtabx, sizeof(int2) * dsz * K);
 	if (e == cudaSuccess) e = cudaMalloc((void **)&t->d_dsymb, sizeof(double) * (size_t)K * K * K * N);
 	if (e == cudaSuccess) e = cudaMalloc((void **)&t->d_ynorm, sizeof(double) * K * N);
 	if (e == cudaSuccess) e = cudaMalloc((void **)&t->d_ll1, sizeof(int2) * nll);
 	if (e == cudaSuccess) e = cudaMemcpy(t->d_dtab, h_dt, sizeof(double) * dsz * K, cudaMemcpyHostToDevice);
+	if (e == cudaSuccess && t->d_dtabx) {
+		cudaStream_t s = sxs_default_stream();
+		e = (cudaError_t)sxsk_fix_dtab(t->d_dtab, t->d_dtabx, (long)(dsz * K), s);
+		sxs_count_launches(1);
+		if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+	}
 	if (e == cudaSuccess) {
 		for (size_t i = 0; i < dsz * K; i++) h_df[i] = (float)h_dt[i];
 		e = cudaMemcpy(t->d_dtabf, h_df, sizeof(float) * dsz * K, cudaMemcpyHostToDevice);
@@ -323,7 +330,7 @@ int sxs_ltables_get(int L, const sxs_ltables **out)
 	if (e == cudaSuccess) e = cudaMemcpy(t->d_ll1, h_ll, sizeof(int2) * nll, cudaMemcpyHostToDevice);
 	free(h_dt); free(h_yn); free(h_ll); free(h_df);
 	if (e != cudaSuccess) {
-		cudaFree(t->d_dtab); cudaFree(t->d_dtabf); cudaFree(t->d_dsymb); cudaFree(t->d_ynorm); cudaFree(t->d_ll1);
+		cudaFree(t->d_dtab); cudaFree(t->d_dtabf); cudaFree(t->d_dtabx); cudaFree(t->d_dsymb); cudaFree(t->d_ynorm); cudaFree(t->d_ll1);
 		free(t);
 		pthread_mutex_unlock(&g_lt_lock);
 		return sxs_cuda_fail(e, "per-L table upload");
