@@ -47,10 +47,11 @@ typedef struct {
 /* A_lm expansion (FP64, the reference's j_l series and Legendre recurrence):
  * per-atom Y_lm and radius into ylm_ws / rad_ws, then one block per (q, l)
  * with the atoms staged through shared memory (series, accumulation, 4 pi
- * i^l phase).  spf_out uses the host flat layout [3][Q][K2][2]. */
+ * i^l phase).  spf_out uses the host flat layout [3][Q][K2][2].  fixed:
+ * accumulation in fixed point (Y_lm as limbs of the same size). */
 int sxsk_expand(const double *xyz, const double *vac, const double *dum, const double *wfac,
                 int natoms, const double *q, int Q, int L, const double *ynorm,
-                double2 *ylm_ws, double *rad_ws, double *spf_out, cudaStream_t s);
+                double2 *ylm_ws, double *rad_ws, double *spf_out, int fixed, cudaStream_t s);
 size_t sxsk_expand_ws_ylm(int natoms, int L);
 size_t sxsk_expand_ws_rad(int natoms);
 int sxsk_expand_launches(void);

@@ -46,58 +46,126 @@ __device__ double sbessel(int l, double x)
 	return l == 0 ? 1.0 : 0.0;
 }
 
+/* |Y_lm| <= sqrt((2l + 1) / 4 pi) < 2^y_exp(l) */
+__device__ __forceinline__ int y_exp(int l) { return l == 0 ? -1 : (l < 6 ? 0 : (l < 25 ? 1 : 2)); }
+
+/* Y_lm as 16 bytes: two doubles, or (fixed-point accumulation) the limbs {re h,
+ * re l, im h, im l} of Y / 2^y_exp = (h 2^27 + l) 2^-54: a sum with 1.5 2^52
+ * leaves the rounded integer in the low word, and the remainder is exact */
+__device__ __forceinline__ void y_store(double2 *o, double re, double im, int) { *o = make_double2(re, im); }
+__device__ __forceinline__ void y_store(int4 *o, double re, double im, int l)
+{
+	const double M = 6755399441055744.0, c = ldexp(1.0, 27 - y_exp(l));
+	double a = __fma_rn(re, c, M), b = __fma_rn(im, c, M);
+	double ar = __fma_rn(re, c, -(a - M)), br = __fma_rn(im, c, -(b - M));
+	*o = make_int4(__double2loint(a), __double2loint(__fma_rn(ar, 134217728.0, M)), __double2loint(b),
+	               __double2loint(__fma_rn(br, 134217728.0, M)));
+}
+
+#define YLM_ATOMS 16
+#define YLM_THREADS 128
+
 /* Per atom and m >= 0: P_l^m(cos theta) by the recurrence of
  * src/borrowed.c:40-65 (N = L+1), times the Y norm, times e^{-i m phi}
- * (src/pdb2spf.c:76-84), written for +m and -m. */
-__global__ void k_ylm(const double *__restrict__ xyz, int natoms, int L, const double *__restrict__ ynorm,
-                      double2 *__restrict__ ylm, double *__restrict__ rad)
+ * (src/pdb2spf.c:76-84), written for +m and -m.  Block = YLM_ATOMS atoms:
+ * one thread per atom takes its angles, then threads take (atom, m); the
+ * recurrence's quotients, which depend on (l, m) alone, are divided once per
+ * block.  Bound by the FP64 pipe (3,500 atoms at L = 20: 0.40 ms with angles,
+ * quotients and phase factors formed per (atom, m) or per l).  The radius of
+ * an atom whose angles are not finite is written as NaN in the limb form,
+ * which cannot hold its Y_lm. */
+template <typename Y, bool LIMBS>
+__global__ void __launch_bounds__(YLM_THREADS)
+k_ylm(const double *__restrict__ xyz, int natoms, int L, const double *__restrict__ ynorm, Y *__restrict__ ylm,
+      double *__restrict__ rad)
 {
-	int K = L + 1, K2 = K * K;
-	long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= (long)natoms * K) return;
-	int a = (int)(t / K), m = (int)(t % K);
-	double x = xyz[3 * a], y = xyz[3 * a + 1], z = xyz[3 * a + 2];
-	double r = sqrt(x * x + y * y + z * z);
-	if (m == 0 && rad) rad[a] = r;
-	double th = acos(z / r);
-	double ph;
-	if (y > 0.0) ph = acos(x / sqrt(x * x + y * y));
-	else ph = -acos(x / sqrt(x * x + y * y)) + 2.0 * SXS_PI;
-	double c = cos(th);
-	double s = sqrt(1. - c * c);
-	int N = K;
-	/* P_m^m: the reference's diagonal chain (lines 54 and 63 agree on the
-	 * formula), then P_{m+1}^m and the upward recurrence in l. */
-	double pmm = 1;
-	for (int j = 1; j <= m; j++) pmm = -1. * (2. * j - 1.) * s * pmm;
-	double p_lm2 = 0.0, p_lm1 = pmm;
-	double2 *out = ylm + (size_t)a * K2;
-	for (int l = m; l < N; l++) {
-		double p;
-		if (l == m) {
-			p = pmm;
-		} else if (l == m + 1) {
-			if (m == 0) p = c;                          /* P_1^0 = x */
-			else p = (2. * m + 1.) * c * pmm;           /* P_{m+1}^m */
-		} else {
-			if (m == 0) p = (2. * l - 1.) / l * c * p_lm1 - (l - 1.) / l * p_lm2;
-			else p = (2. * l - 1.) / (l - m) * c * p_lm1 - (l + m - 1.) / (l - m) * p_lm2;
-		}
-		p_lm2 = p_lm1;
-		p_lm1 = p;
-		if (l == m) { p_lm2 = 0.0; p_lm1 = p; }
-		double hp = ynorm[l * (2 * L + 1) + (m + L)] * p;
-		out[lm_index(l, m)] = make_double2(hp * cos(ph * m), hp * sin(-ph * m));
-		if (m > 0) {
-			double hn = ynorm[l * (2 * L + 1) + (-m + L)] * p;
-			out[lm_index(l, -m)] = make_double2(hn * cos(ph * (-m)), hn * sin(-ph * (-m)));
+	extern __shared__ double2 quo[];           /* [L (L + 1) / 2]: (2l - 1) / (l - m), (l + m - 1) / (l - m) */
+	__shared__ double ang[YLM_ATOMS][3];       /* cos theta, sin theta, phi */
+	int K = L + 1, K2 = K * K, N = K;
+	int a0 = blockIdx.x * YLM_ATOMS, na = min(YLM_ATOMS, natoms - a0);
+	for (int i = threadIdx.x; i < K * K; i += YLM_THREADS) {
+		int m = i / K, l = i % K;
+		if (l > m + 1) quo[l * (l - 1) / 2 + m] = make_double2((2. * l - 1.) / (l - m), (l + m - 1.) / (l - m));
+	}
+	if (threadIdx.x < na) {
+		int a = a0 + threadIdx.x;
+		double x = xyz[3 * a], y = xyz[3 * a + 1], z = xyz[3 * a + 2];
+		double r = sqrt(x * x + y * y + z * z);
+		double th = acos(z / r);
+		double ph;
+		if (y > 0.0) ph = acos(x / sqrt(x * x + y * y));
+		else ph = -acos(x / sqrt(x * x + y * y)) + 2.0 * SXS_PI;
+		rad[a] = LIMBS && !(isfinite(th) && isfinite(ph)) ? nan("") : r;
+		double c = cos(th);
+		ang[threadIdx.x][0] = c;
+		ang[threadIdx.x][1] = sqrt(1. - c * c);
+		ang[threadIdx.x][2] = ph;
+	}
+	__syncthreads();
+	for (int i = threadIdx.x; i < na * K; i += YLM_THREADS) {
+		int m = i / na, ai = i % na;
+		double c = ang[ai][0], s = ang[ai][1], ph = ang[ai][2];
+		/* P_m^m: the reference's diagonal chain (lines 54 and 63 agree on the
+		 * formula), then P_{m+1}^m and the upward recurrence in l. */
+		double pmm = 1;
+		for (int j = 1; j <= m; j++) pmm = -1. * (2. * j - 1.) * s * pmm;
+		double p_lm2 = 0.0, p_lm1 = pmm;
+		/* the phase factors do not depend on l; those of -m are the conjugates */
+		double cp = cos(ph * m), sp = sin(-ph * m);
+		Y *out = ylm + (size_t)(a0 + ai) * K2;
+		for (int l = m; l < N; l++) {
+			double p;
+			if (l == m) {
+				p = pmm;
+			} else if (l == m + 1) {
+				if (m == 0) p = c;                          /* P_1^0 = x */
+				else p = (2. * m + 1.) * c * pmm;           /* P_{m+1}^m */
+			} else {
+				double2 f = quo[l * (l - 1) / 2 + m];
+				p = f.x * c * p_lm1 - f.y * p_lm2;
+			}
+			p_lm2 = p_lm1;
+			p_lm1 = p;
+			if (l == m) { p_lm2 = 0.0; p_lm1 = p; }
+			double hp = ynorm[l * (2 * L + 1) + (m + L)] * p;
+			y_store(out + lm_index(l, m), hp * cp, hp * sp, l);
+			if (m > 0) {
+				double hn = ynorm[l * (2 * L + 1) + (-m + L)] * p;
+				y_store(out + lm_index(l, -m), hn * cp, hn * -sp, l);
+			}
 		}
 	}
 }
 
-/* series terms whose divisor (2k)(2k + 2l + 1) and its reciprocal a block
- * of k_expand_ql stages for its l */
+/* series terms whose divisor (2k)(2k + 2l + 1) a block of k_expand_ql keeps
+ * in a table for its l */
 #define EXP_KTAB 128
+
+/* a series divisor D, 2^(bits - 1) < D < 2^bits: itself and 1 / D rounded to
+ * nearest, and inv = floor(2^(63 + bits) / D) */
+struct SeriesDiv {
+	double den, rcp;
+	unsigned long long inv;
+	int bits, pad;
+};
+
+__device__ __forceinline__ SeriesDiv series_div(int k, int l)
+{
+	SeriesDiv d;
+	unsigned long long D = 2ull * k * (2ull * k + 2ull * l + 1ull);   /* never a power of two: it has an odd factor */
+	d.den = (double)D;
+	d.rcp = 1.0 / d.den;
+	d.bits = 64 - __clzll((long long)D);
+	unsigned long long q = (1ull << 63) / D, r = (1ull << 63) - q * D;
+	for (int i = 0; i < d.bits; i++) {
+		r <<= 1;
+		q = 2 * q + (r >= D);
+		if (r >= D) r -= D;
+	}
+	d.inv = q;
+	d.pad = 0;
+	return d;
+}
 
 /* num / den, correctly rounded, for an integer den > 0 with y = 1/den
  * rounded to nearest and |num| a normal number: q0 = num y, the remainder
@@ -114,55 +182,126 @@ __device__ __forceinline__ double div_by_int(double num, double den, double y)
 	return fma(r, y, q0);
 }
 
-/* j_l(x) with the series of sbessel and the same value: the same terms in
- * the same order, with three changes that leave the rounded series alone.
- * The stop test fabs(term / sum) > 1e-5 is decided by comparing |term|
- * with |sum| 1e-5 (1 +- 1e-10), whose rounding errors are far below that
- * margin; only a quotient within the margin is divided out.  The ratio of
- * consecutive terms, -x^2 / ((2k)(2k + 2l + 1)), is divided as above with
- * the block's table dk[k] = {(2k)(2k + 2l + 1), its reciprocal} for k <
- * EXP_KTAB.  x^l is a chain of products instead of pow (a few ulps,
- * outside the cancelling sum).  term0 = 1 / (2l+1)!! is the block's. */
-__device__ __forceinline__ double sbessel_fast(int l, double x, double term0, const double2 *dk)
+/* -|num| / D, correctly rounded, in integers: mant = the 53-bit significand
+ * of num at the top of 64 bits, en its exponent field.  R = floor(mant inv /
+ * 2^64) is less than 2 below the quotient (scaled to [2^62, 2^64)), whose 53
+ * leading bits are rounded to nearest; there are no ties (a quotient of a
+ * 53-bit number by D has at most 53 bits or infinitely many), so only the
+ * remainder one below the half is not decided (open). */
+__device__ __forceinline__ double series_ratio(unsigned long long mant, int en, unsigned long long inv, int bits, bool &open)
 {
-	if (x > 0.0) {
-		double tl1 = 2.0 * (double)l + 1.0;
-		double num = (-1.0) * x * x;
-		double term = term0, sum = term0;
-		const double c = 0.00001, hi = c * (1.0 + 1e-10), lo = c * (1.0 - 1e-10);
-		bool tiny = fabs(num) < 0x1p-900;   /* keep the division where num is near the subnormals */
-		for (int k = 1; k < 100000; k++) {
-			double at = fabs(term), as = fabs(sum);
-			bool go;
-			if (at > as * hi) go = true;
-			else if (at < as * lo) go = false;
-			else go = fabs(term / sum) > c;
-			if (!go) break;
-			double ratio;
-			if (k < EXP_KTAB && !tiny) {
-				double2 d = dk[k];
-				ratio = div_by_int(num, d.x, d.y);
-			} else {
-				ratio = num / ((2.0 * (double)k) * (2.0 * (double)k + tl1));
-			}
-			term = term * ratio;
-			sum = sum + term;
-		}
-		double xl = 1.0;
-		for (int i = 0; i < l; i++) xl = xl * x;
-		return sum * xl;
+	unsigned long long R = __umul64hi(mant, inv);
+	int big = (int)(R >> 63), sh = 10 + big;
+	unsigned half = 512u << big, low = (unsigned)R & (2 * half - 1);
+	open = low == half - 1;
+	unsigned long long S = (R >> sh) + (low >= half);
+	return __longlong_as_double((long long)((((unsigned long long)(unsigned)(en - bits + big + 2047) << 52) + S)));
+}
+
+/* the rare exact forms, kept out of line so that no part of their divisions
+ * is issued ahead of need */
+__device__ __noinline__ bool series_goes_on(double term, double sum) { return fabs(term / sum) > 0.00001; }
+__device__ __noinline__ double series_sum(int l, double x, double term0)
+{
+	double tl1 = 2.0 * (double)l + 1.0, term = term0, sum = term0;
+	for (int k = 1; fabs(term / sum) > 0.00001 && k < 100000; k++) {
+		double ratio = ((-1.0) * x * x) / ((2.0 * (double)k) * (2.0 * (double)k + tl1));
+		term = term * ratio;
+		sum = sum + term;
 	}
-	return l == 0 ? 1.0 : 0.0;
+	return sum;
+}
+
+/* j_l(x) with the series of sbessel and the same sum: the same terms in the
+ * same order, the product and the sum of each term on the FP64 pipe (2
+ * operations of 73 clocks per warp and scheduler) and the rest beside it: the
+ * ratio of consecutive terms, -x^2 / ((2k)(2k + 2l + 1)), in integers as above
+ * with the block's table for k < EXP_KTAB, and the stop test fabs(term /
+ * sum) > 1e-5 on the leading 20 bits of both (as floats relative to term0's
+ * exponent), with the quotient only where those do not decide.  x^l is formed
+ * by squaring (SQ) or as a chain of products, a few ulps, outside the
+ * cancelling sum.  term0 = 1 / (2l+1)!! is the block's.  Two or four series
+ * per thread at once measured slower (registers). */
+template <bool SQ>
+__device__ __forceinline__ double sbessel_fast(int l, double x, double term0, const SeriesDiv *dk)
+{
+	if (!(x > 0.0)) return l == 0 ? 1.0 : 0.0;
+	double num = (-1.0) * x * x, term = term0, sum = term0;
+	unsigned long long nb = (unsigned long long)__double_as_longlong(num);
+	int en = (int)(nb >> 52) & 0x7ff;
+	unsigned long long mant = (nb << 11) | 0x8000000000000000ull;
+	int off = (__double2hiint(term0) & 0x7ff00000) - (127 << 20);
+	bool slow = en <= 123 || en >= 1923;   /* |num| outside 2^+-900: quotients may be subnormal */
+	for (int k = 1; !slow; k++) {
+		int ht = (__double2hiint(term) & 0x7fffffff) - off, hs = (__double2hiint(sum) & 0x7fffffff) - off;
+		float tf = __int_as_float(ht << 3), sf = __int_as_float(hs << 3) * 1e-5f;
+		bool in = (unsigned)(ht - (20 << 20)) < (unsigned)(234 << 20) && (unsigned)(hs - (20 << 20)) < (unsigned)(234 << 20);
+		if (in && tf < sf * 0.99999f) break;
+		if (!(in && tf > sf * 1.00001f) && !series_goes_on(term, sum)) break;
+		if (k == EXP_KTAB) {
+			slow = true;
+			break;
+		}
+		bool open;
+		double ratio = series_ratio(mant, en, dk[k].inv, dk[k].bits, open);
+		if (open) ratio = div_by_int(num, dk[k].den, dk[k].rcp);
+		term = term * ratio;
+		sum = sum + term;
+	}
+	if (slow) sum = series_sum(l, x, term0);
+	double xl = 1.0;
+	if (SQ) {
+		double b = x;
+		for (int e = l; e; e >>= 1) {
+			if (e & 1) xl = xl * b;
+			if (e > 1) b = b * b;
+		}
+	} else {
+		for (int i = 0; i < l; i++) xl = xl * x;
+	}
+	return sum * xl;
 }
 
 #define EXP_THREADS 128
+/* atoms staged at a time by the fixed-point form: 512 products of its limbs
+ * fit in 63 bits */
+#define EXP_CHUNK 512
+
+/* (double)v in two FP64 operations: each word under an exponent of its own */
+__device__ __forceinline__ double to_double(long long v)
+{
+	double hi = __hiloint2double(0x45300000, (int)((unsigned)(v >> 32) ^ 0x80000000u));
+	double lo = __hiloint2double(0x43300000, (int)(unsigned)v);
+	return (hi - (0x1p84 + 0x1p63 + 0x1p52)) + lo;
+}
+/* 2^e for a normal result */
+__device__ __forceinline__ double exp2i(int e)
+{
+	return __longlong_as_double((long long)(unsigned)(e + 1023) << 52);
+}
+
+/* 4 pi i^l times the sums of the block's (q, l): thread t < 2l + 1 writes m =
+ * t - l of the three channels */
+__device__ __forceinline__ void expand_write(double *spf, const double *v, int iq, int l, int t, int Q, int K2)
+{
+	const double fp = 4.0 * SXS_PI;
+	double cre[4] = {fp, 0.0, -fp, 0.0}, cim[4] = {0.0, fp, 0.0, -fp};
+	double c_r = cre[l % 4], c_i = cim[l % 4];
+	size_t chs = (size_t)Q * K2 * 2;
+	double *o = spf + ((size_t)iq * K2 + l * l + t) * 2;
+	o[0] = c_r * v[0] - c_i * v[1];           o[1] = c_r * v[1] + c_i * v[0];
+	o[chs] = c_r * v[2] - c_i * v[3];         o[chs + 1] = c_r * v[3] + c_i * v[2];
+	o[2 * chs] = c_r * v[4] - c_i * v[5];     o[2 * chs + 1] = c_r * v[5] + c_i * v[4];
+}
 
 /* A[ch][q][l m] for one (q, l) per block: atoms in tiles of EXP_THREADS,
  * staged through shared memory as w_ch = f_ch(a) j_l(q r_a) (one series
  * per thread), then accumulated against Y*_lm(a) by (m, slice) threads,
  * each slice a fixed residue class of the tile's atoms; the slices are
  * summed in order and the 4 pi i^l phase applied (src/pdb2spf.c:104-147).
- * Deterministic: the same partition and order on every run. */
+ * Deterministic: the same partition and order on every run.  The exact
+ * scoring's L-BFGS-B fit runs on this form, whose last bits it would
+ * amplify if they moved. */
 __global__ void __launch_bounds__(EXP_THREADS) k_expand_ql(const double2 *__restrict__ ylm,
                                                             const double *__restrict__ rad,
                                                             const double *__restrict__ vac,
@@ -173,6 +312,7 @@ __global__ void __launch_bounds__(EXP_THREADS) k_expand_ql(const double2 *__rest
 {
 	__shared__ double w[3][EXP_THREADS];
 	__shared__ double red[EXP_THREADS][6];
+	__shared__ SeriesDiv dk[EXP_KTAB];
 	int K = L + 1, K2 = K * K;
 	int iq = blockIdx.x / K, l = blockIdx.x % K;
 	int nm = 2 * l + 1, nslice = EXP_THREADS / nm;
@@ -181,18 +321,15 @@ __global__ void __launch_bounds__(EXP_THREADS) k_expand_ql(const double2 *__rest
 	bool acc_thread = sl < nslice;
 	double qv = q[iq];
 	double term0 = 1.0 / odd_factorial(2 * l + 1);
-	__shared__ double2 dk[EXP_KTAB];
-	for (int k = t; k < EXP_KTAB; k += blockDim.x) {
-		double den = (2.0 * (double)k) * (2.0 * (double)k + (2.0 * (double)l + 1.0));
-		dk[k] = make_double2(den, k > 0 ? 1.0 / den : 0.0);
-	}
+	for (int k = t; k < EXP_KTAB; k += blockDim.x)
+		if (k) dk[k] = series_div(k, l);
 	__syncthreads();
 	double a6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 	const double2 *yl = ylm + l * l;   /* this l's first (l, m) of every atom row */
 	for (int a0 = 0; a0 < natoms; a0 += EXP_THREADS) {
 		int a = a0 + t;
 		if (a < natoms) {
-			double j = sbessel_fast(l, qv * rad[a], term0, dk);
+			double j = sbessel_fast<false>(l, qv * rad[a], term0, dk);
 			w[0][t] = vac[a] * j;
 			w[1][t] = dum[a] * j;
 			w[2][t] = wfac[a] * j;
@@ -217,15 +354,129 @@ __global__ void __launch_bounds__(EXP_THREADS) k_expand_ql(const double2 *__rest
 		double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 		for (int sidx = 0; sidx < nslice; sidx++)
 			for (int c = 0; c < 6; c++) v[c] = v[c] + red[sidx * nm + t][c];
-		const double fp = 4.0 * SXS_PI;
-		double cre[4] = {fp, 0.0, -fp, 0.0}, cim[4] = {0.0, fp, 0.0, -fp};
-		double c_r = cre[l % 4], c_i = cim[l % 4];
-		size_t chs = (size_t)Q * K2 * 2;
-		double *o = spf + ((size_t)iq * K2 + l * l + t) * 2;
-		o[0] = c_r * v[0] - c_i * v[1];           o[1] = c_r * v[1] + c_i * v[0];
-		o[chs] = c_r * v[2] - c_i * v[3];         o[chs + 1] = c_r * v[3] + c_i * v[2];
-		o[2 * chs] = c_r * v[4] - c_i * v[5];     o[2 * chs + 1] = c_r * v[5] + c_i * v[4];
+		expand_write(spf, v, iq, l, t, Q, K2);
 	}
+}
+
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c)
+{
+	long long r;
+	asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+	return r;
+}
+
+/* The same sums with the accumulation in fixed point, off the FP64 pipe,
+ * which the series then has to itself.  Atoms in chunks of EXP_CHUNK: the
+ * weights w_ch, scaled by the largest exponent in the chunk to 53-bit
+ * integers h 2^27 + l, times the limbs of Y (h 2^27 + l, 54 bits) as three
+ * 32 x 32 + 64-bit multiply-adds (h h', and h l' + l h'), sums exact; a
+ * chunk's sums are added to the thread's in double.  Bound by the FP64 pipe:
+ * 2 operations per series term (8.4 terms on average, the longest of each
+ * warp) and ~16 more per (atom, q, l), beside 18 IMAD.WIDE (~83 clocks) per
+ * (atom, l, m); the FP64 form had 9 per term and 6 per (atom, l, m).  the
+ * whole call (with k_ylm and one stream-ordered work buffer) 3,500 atoms, L =
+ * 20, Q = 101: 4.9 -> 1.4 ms; 8,000, L = 30, Q = 201: 36.2 -> 9.9.
+ * Blocks per SM (10: 48 registers, some spilled outside the loops): whole
+ * call 1.54 / 11.1 ms with 7, 1.39 / 9.9 with 9, 1.31 / 8.9 with 10, 1.72 /
+ * 11.8 with 11. */
+__global__ void __launch_bounds__(EXP_THREADS, 10) k_expand_fix(const int4 *__restrict__ ylm,
+                                                             const double *__restrict__ rad,
+                                                             const double *__restrict__ vac,
+                                                             const double *__restrict__ dum,
+                                                             const double *__restrict__ wfac, int natoms,
+                                                             const double *__restrict__ q, int Q, int L,
+                                                             double *__restrict__ spf)
+{
+	__shared__ long long w[3][EXP_CHUNK];   /* the weights' bits, then their limbs; the slices' sums at the end */
+	__shared__ SeriesDiv dk[EXP_KTAB];
+	__shared__ int emax[3];
+	int K = L + 1, K2 = K * K;
+	int iq = blockIdx.x / K, l = blockIdx.x % K;
+	int nm = 2 * l + 1, nslice = EXP_THREADS / nm;
+	int t = threadIdx.x;
+	int mi = t % nm, sl = t / nm;
+	bool acc_thread = sl < nslice;
+	double qv = q[iq];
+	double term0 = 1.0 / odd_factorial(2 * l + 1);
+	for (int k = t; k < EXP_KTAB; k += blockDim.x)
+		if (k) dk[k] = series_div(k, l);
+	if (t < 3) emax[t] = 0;
+	__syncthreads();
+	double a6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+	const int4 *yl = ylm + l * l + mi;   /* this thread's (l, m) of every atom row */
+	for (int a0 = 0; a0 < natoms; a0 += EXP_CHUNK) {
+		int na = min(EXP_CHUNK, natoms - a0);
+		int em[3] = {0, 0, 0};
+		for (int k = t; k < na; k += EXP_THREADS) {
+			int a = a0 + k;
+			double r = rad[a], j = sbessel_fast<true>(l, qv * r, term0, dk);
+			if (isnan(r)) j = r;
+			double v[3] = {vac[a] * j, dum[a] * j, wfac[a] * j};
+#pragma unroll
+			for (int c = 0; c < 3; c++) {
+				w[c][k] = __double_as_longlong(v[c]);
+				em[c] = max(em[c], (__double2hiint(v[c]) >> 20) & 0x7ff);
+			}
+		}
+#pragma unroll
+		for (int c = 0; c < 3; c++) {
+			int v = __reduce_max_sync(0xffffffffu, em[c]);
+			if (t % 32 == 0) atomicMax(&emax[c], v);
+		}
+		__syncthreads();
+		for (int c = 0; c < 3; c++) em[c] = emax[c];
+		/* w = M 2^(E - 1075) -> M >> (emax - E), rounded: unit 2^(emax - 1075) */
+		for (int k = t; k < na; k += EXP_THREADS)
+#pragma unroll
+			for (int c = 0; c < 3; c++) {
+				long long b = w[c][k];
+				int E = (int)(b >> 52) & 0x7ff, s = em[c] - E;
+				long long M = (b & 0xfffffffffffffll) | 0x10000000000000ll;
+				M = E == 0 || s > 53 ? 0 : (s > 0 ? (M + (1ll << (s - 1))) >> s : M);
+				if (b < 0) M = -M;
+				int h = (int)((M + (1ll << 26)) >> 27), lo = (int)((unsigned)M - ((unsigned)h << 27));
+				w[c][k] = (long long)(((unsigned long long)(unsigned)lo << 32) | (unsigned)h);
+			}
+		__syncthreads();
+		if (t < 3) emax[t] = 0;
+		if (acc_thread) {
+			long long hh[6] = {0, 0, 0, 0, 0, 0}, mid[6] = {0, 0, 0, 0, 0, 0};
+			for (int k = sl; k < na; k += nslice) {
+				int4 y = __ldg(yl + (size_t)(a0 + k) * K2);
+#pragma unroll
+				for (int c = 0; c < 3; c++) {
+					long long b = w[c][k];
+					int wh = (int)b, wl = (int)(b >> 32);
+					hh[2 * c] = mad_wide(wh, y.x, hh[2 * c]);
+					hh[2 * c + 1] = mad_wide(wh, y.z, hh[2 * c + 1]);
+					mid[2 * c] = mad_wide(wh, y.y, mid[2 * c]);
+					mid[2 * c + 1] = mad_wide(wh, y.w, mid[2 * c + 1]);
+					mid[2 * c] = mad_wide(wl, y.x, mid[2 * c]);
+					mid[2 * c + 1] = mad_wide(wl, y.z, mid[2 * c + 1]);
+				}
+			}
+#pragma unroll
+			for (int c = 0; c < 6; c++) {
+				/* hh 2^54 + mid 2^27 in units of 2^(emax - 1075) 2^(y_exp - 54) */
+				int e = em[c / 2], s2 = e - 1075 + y_exp(l);
+				double u = e == 0x7ff ? nan("") : (s2 > -1022 ? exp2i(s2) : 0.0);
+				a6[c] = fma(to_double(hh[c] + ((mid[c] + (1 << 26)) >> 27)), u, a6[c]);
+			}
+		}
+		__syncthreads();
+	}
+	double *red = reinterpret_cast<double *>(&w[0][0]);   /* [EXP_THREADS][6] */
+	if (acc_thread)
+		for (int c = 0; c < 6; c++) red[t * 6 + c] = a6[c];
+	__syncthreads();
+	double *tot = red + EXP_THREADS * 6;                   /* [2l + 1][6] */
+	for (int i = t; i < 6 * nm; i += EXP_THREADS) {
+		double v = 0.0;
+		for (int sidx = 0; sidx < nslice; sidx++) v = v + red[sidx * nm * 6 + i];
+		tot[i] = v;
+	}
+	__syncthreads();
+	if (t < nm) expand_write(spf, tot + 6 * t, iq, l, t, Q, K2);
 }
 
 /* bes[iz][p][q] = j_p(z q) (src/fftsaxs.c:110-121), q fastest. */
@@ -421,7 +672,7 @@ size_t sxsk_expand_ws_rad(int natoms) { return (size_t)natoms * sizeof(double); 
 
 int sxsk_expand(const double *xyz, const double *vac, const double *dum, const double *wfac, int natoms,
                  const double *q, int Q, int L, const double *ynorm, double2 *ylm_ws, double *rad_ws,
-                 double *spf_out, cudaStream_t s)
+                 double *spf_out, int fixed, cudaStream_t s)
 {
 	int K = L + 1;
 	if (natoms <= 0) {
@@ -429,8 +680,14 @@ int sxsk_expand(const double *xyz, const double *vac, const double *dum, const d
 		return cudaGetLastError();
 	}
 	if ((long)Q * K > 0x7fffffffL) return cudaErrorInvalidValue;
-	k_ylm<<<nblk((long)natoms * K, 128), 128, 0, s>>>(xyz, natoms, L, ynorm, ylm_ws, rad_ws);
-	k_expand_ql<<<Q * K, EXP_THREADS, 0, s>>>(ylm_ws, rad_ws, vac, dum, wfac, natoms, q, Q, L, spf_out);
+	size_t qsm = sizeof(double2) * (size_t)K * L / 2;   /* at most 29 KB (L = 60) */
+	if (fixed) {
+		k_ylm<int4, true><<<nblk(natoms, YLM_ATOMS), YLM_THREADS, qsm, s>>>(xyz, natoms, L, ynorm, (int4 *)ylm_ws, rad_ws);
+		k_expand_fix<<<Q * K, EXP_THREADS, 0, s>>>((const int4 *)ylm_ws, rad_ws, vac, dum, wfac, natoms, q, Q, L, spf_out);
+	} else {
+		k_ylm<double2, false><<<nblk(natoms, YLM_ATOMS), YLM_THREADS, qsm, s>>>(xyz, natoms, L, ynorm, ylm_ws, rad_ws);
+		k_expand_ql<<<Q * K, EXP_THREADS, 0, s>>>(ylm_ws, rad_ws, vac, dum, wfac, natoms, q, Q, L, spf_out);
+	}
 	return cudaGetLastError();
 }
 
@@ -571,7 +828,7 @@ extern "C" int sxsg_expand_noalloc(const double *xyz, const double *vac, const d
 		if (e != cudaSuccess) return (int)e;
 		w = base + off_w;
 	}
-	int rc = sxsk_expand(xyz, vac, dum, w, natoms, q, Q, L, base, (double2 *)(base + off_y), base + off_r, spf_out, s);
+	int rc = sxsk_expand(xyz, vac, dum, w, natoms, q, Q, L, base, (double2 *)(base + off_y), base + off_r, spf_out, 1, s);
 	sxs_count_launches(natoms > 0 ? sxsk_expand_launches() : 0);
 	return rc;
 }

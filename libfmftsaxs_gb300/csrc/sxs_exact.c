@@ -114,7 +114,7 @@ int sxsg_score_exact(const double *rec_xyz, int nrec, const double *lig_xyz, int
 		e = cudaMemcpyAsync(d_xyz, h_xyz, sizeof(double) * 3 * na * (size_t)nb, cudaMemcpyHostToDevice, s);
 		for (int k = 0; k < nb && !e; k++)
 			e = (cudaError_t)sxsk_expand(d_xyz + 3 * (size_t)na * k, d_vac, d_dum, d_wf, na, d_q, Q, L, lt->d_ynorm,
-			                             d_ylm, d_rad, d_spf + spf_n * k, s);
+			                             d_ylm, d_rad, d_spf + spf_n * k, 0, s);
 		if (!e) e = (cudaError_t)sxsk_self_cross(d_spf, nb, Q, L, d_cross, s);
 		if (!e)
 			e = (cudaError_t)sxs_fit_lbfgsb_launch(d_cross, 0, nb, Q, d_q, d_a, mult, 1.0, 0, d_chi, d_c1, d_c2, NULL,

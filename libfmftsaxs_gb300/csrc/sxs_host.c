@@ -131,18 +131,23 @@ int sxsg_expand(const double *xyz, const double *vac, const double *dum, const d
 	double *wf = malloc(sizeof(double) * (natoms > 0 ? natoms : 1));
 	if (!wf) return sxs_fail(-5, "out of host memory");
 	for (int i = 0; i < natoms; i++) wf[i] = sasa ? water_ff * sasa[i] : 0.0;
-	double *d_xyz = NULL, *d_vac = NULL, *d_dum = NULL, *d_wf = NULL, *d_q = NULL, *d_rad = NULL, *d_out = NULL;
-	double2 *d_ylm = NULL;
-	int na = natoms > 0 ? natoms : 1;
-	cudaError_t e = cudaSuccess;
-	if (!e) e = cudaMalloc((void **)&d_xyz, sizeof(double) * 3 * na);
-	if (!e) e = cudaMalloc((void **)&d_vac, sizeof(double) * na);
-	if (!e) e = cudaMalloc((void **)&d_dum, sizeof(double) * na);
-	if (!e) e = cudaMalloc((void **)&d_wf, sizeof(double) * na);
-	if (!e) e = cudaMalloc((void **)&d_q, sizeof(double) * Q);
-	if (!e) e = cudaMalloc((void **)&d_rad, sxsk_expand_ws_rad(na));
-	if (!e) e = cudaMalloc((void **)&d_ylm, sxsk_expand_ws_ylm(na, L));
-	if (!e) e = cudaMalloc((void **)&d_out, sizeof(double) * spf_n);
+	/* one stream-ordered block for the call: the pool keeps it for the next
+	 * one, where nine device allocations and releases each synchronised
+	 * (1.0 of 2.8 ms at 3,500 atoms, L = 20, Q = 101) */
+	size_t na = natoms > 0 ? (size_t)natoms : 1, off = 0, o[8];
+	const size_t bytes[8] = {sizeof(double) * 3 * na, sizeof(double) * na, sizeof(double) * na, sizeof(double) * na,
+	                         sizeof(double) * Q, sxsk_expand_ws_rad((int)na), sxsk_expand_ws_ylm((int)na, L),
+	                         sizeof(double) * spf_n};
+	for (int i = 0; i < 8; i++) {
+		o[i] = off;
+		off += (bytes[i] + 255) / 256 * 256;
+	}
+	char *ws = NULL;
+	cudaError_t e = cudaMallocAsync((void **)&ws, off, s);
+	double *d_xyz = (double *)(ws + o[0]), *d_vac = (double *)(ws + o[1]), *d_dum = (double *)(ws + o[2]);
+	double *d_wf = (double *)(ws + o[3]), *d_q = (double *)(ws + o[4]), *d_rad = (double *)(ws + o[5]);
+	double2 *d_ylm = (double2 *)(ws + o[6]);
+	double *d_out = (double *)(ws + o[7]);
 	if (!e && natoms > 0) {
 		e = cudaMemcpyAsync(d_xyz, xyz, sizeof(double) * 3 * natoms, cudaMemcpyHostToDevice, s);
 		if (!e) e = cudaMemcpyAsync(d_vac, vac, sizeof(double) * natoms, cudaMemcpyHostToDevice, s);
@@ -151,13 +156,12 @@ int sxsg_expand(const double *xyz, const double *vac, const double *dum, const d
 	}
 	if (!e) e = cudaMemcpyAsync(d_q, q, sizeof(double) * Q, cudaMemcpyHostToDevice, s);
 	if (!e) {
-		e = (cudaError_t)sxsk_expand(d_xyz, d_vac, d_dum, d_wf, natoms, d_q, Q, L, lt->d_ynorm, d_ylm, d_rad, d_out, s);
+		e = (cudaError_t)sxsk_expand(d_xyz, d_vac, d_dum, d_wf, natoms, d_q, Q, L, lt->d_ynorm, d_ylm, d_rad, d_out, 1, s);
 		sxs_count_launches(natoms > 0 ? sxsk_expand_launches() : 0);
 	}
 	if (!e) e = cudaMemcpyAsync(spf_out, d_out, sizeof(double) * spf_n, cudaMemcpyDeviceToHost, s);
+	if (ws) cudaFreeAsync(ws, s);
 	if (!e) e = cudaStreamSynchronize(s);
-	cudaFree(d_xyz); cudaFree(d_vac); cudaFree(d_dum); cudaFree(d_wf); cudaFree(d_q);
-	cudaFree(d_rad); cudaFree(d_ylm); cudaFree(d_out);
 	free(wf);
 	if (e) return sxs_cuda_fail(e, "sxsg_expand");
 	return 0;
