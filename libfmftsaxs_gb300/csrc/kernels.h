@@ -10,7 +10,7 @@
  *   dtab  [K b][K l][N m+L][N m1+L]            Wigner small-d per beta_b = b*pi/L
  *   dsymb [K2 lm][K l1][N p]
  *   bes   [nz][N p][Q]
- *   tau   [NT][nz][K m][K l][K l1][QT]         T^m_{l l1} = i^{l+l1} tau (real)
+ *   tau   [NT][nz][K m][K l][K l1][QT]         T^m_{l l1} = i^{l+l1} tau (real; l, l1 >= m)
  *   rot   [NT][K*N (b,g)][NP pair][3 ch][QT]   pair = (m >= 0, l >= m), m-major (S)
  *   trans [NT][ncombo][NP pair][3 ch][QT]      (S)
  *   cross [npose][6][Q]                        (double)
@@ -71,13 +71,12 @@ int sxsk_sasa(const double *xyz, const double *rad, int n, double probe, const d
 /* j_p(q z) for p in [0,2L]: bes[nz][N][Q] (faithful series) */
 int sxsk_bessel_z(const double *z, int nz, const double *q, int Q, int L, double *bes, cudaStream_t s);
 
-/* translation matrix T^m_{l l1}(q z) = i^{l+l1} tau -> tau; ll1 lists the
- * (l, l1 >= l) pairs */
+/* translation matrix T^m_{l l1}(q z) = i^{l+l1} tau -> tau in one of three
+ * forms: double, float, or int2 limbs of tau / nu2 (kernels_fixed.cu; nu2
+ * from sxsk_fix_nu); ll1 lists the (l, l1 >= l) pairs in the order of l */
+enum { SXSK_TAU_FP64 = 0, SXSK_TAU_FP32 = 1, SXSK_TAU_FIXED = 2 };
 int sxsk_tmatrix(const double *bes, const double *dsymb, int nz, int Q, int L, const int2 *ll1, int nll1,
-                 double *tau, cudaStream_t s);
-
-/* b[i] = (float)a[i] */
-int sxsk_to_float(const double *a, float *b, long n, cudaStream_t s);
+                 const double *nu2, void *tau, int form, cudaStream_t s);
 
 /* self terms cst[6][Q] (already times {1,2,2,1,2,1}); A, B in the host flat layout */
 int sxsk_const_int(const double *A, const double *B, int Q, int L, double *cst, cudaStream_t s);
@@ -106,13 +105,12 @@ size_t sxsk_rotate_tc_scratch(int L);
  * are limbs {re h, re l, im h, im l} (int4), scaled per molecule and q.
  * molecule: sc[2][Qp] (Qp = Q rounded up to 8) = {2^(28 - e), 2^e} of the
  * flat coefficients, spf [3][K2][Q] their limbs (conjugated when conj);
- * two launches.  dtab: limbs of a Wigner-d table.  tau: in place, the FP64
- * matrices to limbs of tau / 2^nu, nu2[nz][Qp] = 2^nu a bound of their norm;
- * two launches. */
+ * two launches.  dtab: limbs of a Wigner-d table.  nu: nu2[nz][Qp] = powers of
+ * two that bound the translation matrices' norms. */
 #define SXSK_FIX_LMAX 31
 int sxsk_fix_molecule(const double *flat, int Q, int L, int conj, double *sc, void *spf, cudaStream_t s);
 int sxsk_fix_dtab(const double *d, int2 *x, long n, cudaStream_t s);
-int sxsk_fix_tau(const double *bes, double *tau, int nz, int Q, int L, double *nu2, cudaStream_t s);
+int sxsk_fix_nu(const double *bes, int nz, int Q, int L, double *nu2, cudaStream_t s);
 int sxsk_fix_rotate(const void *spf, const int2 *dtab, const double2 *tw, int Q, int L, void *out, cudaStream_t s);
 /* as sxsk_translate and sxsk_pose_cross; combo_zbg = the chunk's combos */
 int sxsk_fix_translate(const void *U, const void *tau, const int32_t *combo_zbg, const int32_t *slices, int nslice,

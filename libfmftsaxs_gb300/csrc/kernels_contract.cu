@@ -1154,12 +1154,6 @@ __global__ void k_pose_scatter(const sxsk_pose *__restrict__ tmp, const int32_t 
 	out[atomicAdd(&pos[k], 1)] = ps;
 }
 
-__global__ void k_to_float(const double *__restrict__ a, float *__restrict__ b, long n)
-{
-	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) b[i] = (float)a[i];
-}
-
 /* Grid fit (src/min_saxs.c:170-188 peak rescale, 261-320 best scale,
  * 391-448 point_score).  For one pose and one (c1, c2) cell the model at q_i
  * is in_i = al_i + c2 be_i + c2^2 ga_i with G_i = c1^3 exp(-mult (c1^2-1) q_i^2),
@@ -1604,13 +1598,6 @@ int sxsk_rotate(const void *spf_t, const void *dtab, const double2 *tw, int Q, i
 	if (L < 0 || L + 1 > SXS_LMAX_K || Q <= 0) return cudaErrorInvalidValue;
 	if (fp32) return rotate_any<float>(spf_t, dtab, tw, Q, L, conj, out, gsel, s);
 	return rotate_any<double>(spf_t, dtab, tw, Q, L, conj, out, gsel, s);
-}
-
-int sxsk_to_float(const double *a, float *b, long n, cudaStream_t s)
-{
-	if (n <= 0) return 0;
-	k_to_float<<<nblk(n, 256), 256, 0, s>>>(a, b, n);
-	return cudaGetLastError();
 }
 
 int sxsk_pose_decode(const int64_t *index, int64_t n, int N, int nb, int nz, sxsk_pose *tmp, int32_t *key,

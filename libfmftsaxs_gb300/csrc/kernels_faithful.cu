@@ -9,6 +9,7 @@
  * order with one rounding per operation, as gcc -std=c11 does on the host.
  */
 #include "kernels.h"
+#include "limbs.cuh"
 
 #include <math.h>
 
@@ -24,26 +25,6 @@ __device__ double odd_factorial(int n)
 	double r = 1.0;
 	for (int i = 1; i <= n; i += 2) r *= (double)i;
 	return r;
-}
-
-/* j_l(x) by the reference's truncated power series (src/sfbessel.c:40-60). */
-__device__ double sbessel(int l, double x)
-{
-	if (x > 0.0) {
-		double tl1 = 2.0 * (double)l + 1.0;
-		double term = 1.0 / odd_factorial((int)tl1);
-		double sum = term;
-		/* the reference has no iteration bound; terms decay factorially, so
-		 * the cap (far above any count the series reaches) only guards
-		 * against non-finite input */
-		for (int k = 1; fabs(term / sum) > 0.00001 && k < 100000; k++) {
-			double ratio = ((-1.0) * x * x) / ((2.0 * (double)k) * (2.0 * (double)k + tl1));
-			term = term * ratio;
-			sum = sum + term;
-		}
-		return sum * pow(x, (double)l);
-	}
-	return l == 0 ? 1.0 : 0.0;
 }
 
 /* |Y_lm| <= sqrt((2l + 1) / 4 pi) < 2^y_exp(l) */
@@ -212,20 +193,17 @@ __device__ __noinline__ double series_sum(int l, double x, double term0)
 	return sum;
 }
 
-/* j_l(x) with the series of sbessel and the same sum: the same terms in the
- * same order, the product and the sum of each term on the FP64 pipe (2
+/* The series of sbessel, x > 0, and the same sum: the same terms in the same
+ * order, the product and the sum of each term on the FP64 pipe (2
  * operations of 73 clocks per warp and scheduler) and the rest beside it: the
  * ratio of consecutive terms, -x^2 / ((2k)(2k + 2l + 1)), in integers as above
  * with the block's table for k < EXP_KTAB, and the stop test fabs(term /
  * sum) > 1e-5 on the leading 20 bits of both (as floats relative to term0's
- * exponent), with the quotient only where those do not decide.  x^l is formed
- * by squaring (SQ) or as a chain of products, a few ulps, outside the
- * cancelling sum.  term0 = 1 / (2l+1)!! is the block's.  Two or four series
- * per thread at once measured slower (registers). */
-template <bool SQ>
-__device__ __forceinline__ double sbessel_fast(int l, double x, double term0, const SeriesDiv *dk)
+ * exponent), with the quotient only where those do not decide.  term0 = 1 /
+ * (2l+1)!! is the block's.  Two or four series per thread at once measured
+ * slower (registers). */
+__device__ __forceinline__ double series_fast(int l, double x, double term0, const SeriesDiv *dk)
 {
-	if (!(x > 0.0)) return l == 0 ? 1.0 : 0.0;
 	double num = (-1.0) * x * x, term = term0, sum = term0;
 	unsigned long long nb = (unsigned long long)__double_as_longlong(num);
 	int en = (int)(nb >> 52) & 0x7ff;
@@ -248,8 +226,16 @@ __device__ __forceinline__ double sbessel_fast(int l, double x, double term0, co
 		term = term * ratio;
 		sum = sum + term;
 	}
-	if (slow) sum = series_sum(l, x, term0);
-	double xl = 1.0;
+	return slow ? series_sum(l, x, term0) : sum;
+}
+
+/* j_l(x): x^l is formed by squaring (SQ) or as a chain of products, a few
+ * ulps, outside the cancelling sum */
+template <bool SQ>
+__device__ __forceinline__ double sbessel_fast(int l, double x, double term0, const SeriesDiv *dk)
+{
+	if (!(x > 0.0)) return l == 0 ? 1.0 : 0.0;
+	double sum = series_fast(l, x, term0, dk), xl = 1.0;
 	if (SQ) {
 		double b = x;
 		for (int e = l; e; e >>= 1) {
@@ -373,7 +359,7 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c)
  * chunk's sums are added to the thread's in double.  Bound by the FP64 pipe:
  * 2 operations per series term (8.4 terms on average, the longest of each
  * warp) and ~16 more per (atom, q, l), beside 18 IMAD.WIDE (~83 clocks) per
- * (atom, l, m); the FP64 form had 9 per term and 6 per (atom, l, m).  the
+ * (atom, l, m); the FP64 form had 9 per term and 6 per (atom, l, m).  The
  * whole call (with k_ylm and one stream-ordered work buffer) 3,500 atoms, L =
  * 20, Q = 101: 4.9 -> 1.4 ms; 8,000, L = 30, Q = 201: 36.2 -> 9.9.
  * Blocks per SM (10: 48 registers, some spilled outside the loops): whole
@@ -479,59 +465,83 @@ __global__ void __launch_bounds__(EXP_THREADS, 10) k_expand_fix(const int4 *__re
 	if (t < nm) expand_write(spf, tot + 6 * t, iq, l, t, Q, K2);
 }
 
-/* bes[iz][p][q] = j_p(z q) (src/fftsaxs.c:110-121), q fastest. */
-__global__ void k_bessel_z(const double *__restrict__ z, int nz, const double *__restrict__ q, int Q, int L,
-                           double *__restrict__ bes)
+/* bes[iz][p][q] = j_p(z q) (src/fftsaxs.c:110-121), q fastest: the
+ * reference's truncated power series (src/sfbessel.c:40-60) times pow(x, p).
+ * Block = one p and 128 (z, q), so that the series divisors are shared (0.077
+ * -> 0.037 ms at L = 20, Q = 101, 16 z). */
+__global__ void __launch_bounds__(128) k_bessel_z(const double *__restrict__ z, int nz, const double *__restrict__ q,
+                                                  int Q, int L, double *__restrict__ bes)
 {
-	int N = 2 * L + 1;
-	long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= (long)nz * Q * N) return;
-	int iq = (int)(t % Q);
-	long r2 = t / Q;
-	int p = (int)(r2 % N), iz = (int)(r2 / N);
-	bes[t] = sbessel(p, z[iz] * q[iq]);
+	__shared__ SeriesDiv dk[EXP_KTAB];
+	int N = 2 * L + 1, nb = (nz * Q + 127) / 128;
+	int p = blockIdx.x / nb, t = blockIdx.x % nb * 128 + threadIdx.x;
+	for (int k = threadIdx.x; k < EXP_KTAB; k += 128)
+		if (k) dk[k] = series_div(k, p);
+	double term0 = 1.0 / odd_factorial(2 * p + 1);
+	__syncthreads();
+	if (t >= nz * Q) return;
+	int iq = t % Q, iz = t / Q;
+	double x = z[iz] * q[iq];
+	bes[((size_t)iz * N + p) * Q + iq] = x > 0.0 ? series_fast(p, x, term0, dk) * pow(x, (double)p) : (p == 0 ? 1.0 : 0.0);
 }
+
+/* forms of tau: double, float, and the limbs of tau / 2^nu (kernels_fixed.cu) */
+__device__ __forceinline__ void tau_store(double *o, double v, double) { *o = v; }
+__device__ __forceinline__ void tau_store(float *o, double v, double) { *o = (float)v; }
+__device__ __forceinline__ void tau_store(int2 *o, double v, double c28) { *o = sxs_limbs(v, c28); }
+
 /* T^{|m|}_{l l1}(q z) = sum_p (-1)^m i^p j_p d_lm(l1,p) for l <= l1, mirrored
- * (src/fftsaxs.c:182-243).  Thread = (iz, m, l, l1 >= l, q), q fastest.
- * Output in the q-tiled layout of the contraction tables (tiles of SXS_QT q).
+ * (src/fftsaxs.c:182-243).  Thread = (iz, m, (m <= l, l1 >= l), q), q fastest;
+ * nbx blocks per (iz, m), those past its pairs return at once.
+ * Output in the q-tiled layout of the contraction tables (tiles of SXS_QT q,
+ * zeros past Q), entries with l, l1 >= m only (no others are read).
  * The 3j factor 3j(l p l1; 0 0 0) vanishes unless l + p + l1 is even, so T
  * is real for even l + l1 and imaginary for odd l + l1 (the other part is
  * the sum of exact zeros and binary128 round-off below 1e-30 relative); the
- * table keeps that one real number, tau = Re T (even) or Im T (odd). */
-__global__ void k_tmatrix(const double *__restrict__ bes, const double *__restrict__ ds, int nz, int Q, int L,
-                          const int2 *__restrict__ ll1, int nll1, double *__restrict__ tau)
+ * table keeps that one real number, tau = Re T (even) or Im T (odd), in the
+ * form that the run's translation reads.
+ * The reference sums Re and Im with i^p in {1, i, -1, -i}; for the component
+ * kept here the terms with p of the other parity add +-0, so summing only p
+ * = l + l1 (mod 2), in the same order, gives the same value bit for bit; the
+ * signs of (-1)^m and i^p are exact and turn the sum into alternate sums and
+ * differences of the products: two FP64 operations per term (four with the
+ * signs multiplied in), 63 % of that pipe's rate at L = 30.  With the float
+ * form written here, not by a pass over a double table, 16 z of the mixed
+ * path take 0.25 + 0.04 -> 0.20 ms at L = 20, Q = 101 and 2.14 + 0.29 -> 1.69
+ * ms at L = 30, Q = 201. */
+template <typename T>
+__global__ void __launch_bounds__(128) k_tmatrix(const double *__restrict__ bes, const double *__restrict__ ds, int nz,
+                                                 int Q, int L, const int2 *__restrict__ ll1, int nll1, int nbx,
+                                                 const double *__restrict__ nu2, T *__restrict__ tau)
 {
-	int K = L + 1, N = 2 * L + 1;
-	long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= (long)nz * (K) * nll1 * Q) return;
-	int iq = (int)(t % Q);
-	long r2 = t / Q;
-	int j = (int)(r2 % nll1);
-	r2 /= nll1;
-	int m = (int)(r2 % K), iz = (int)(r2 / K);
-	int l = ll1[j].x, l1 = ll1[j].y;
-	if (l < m) return;
-	double sgn = (m % 2 == 0) ? 1.0 : -1.0;
-	const double *dp = ds + ((size_t)lm_index(l, m) * K + l1) * N;
-	const double *bp = bes + (size_t)iz * N * Q + iq;
-	/* the reference sums Re and Im with i^p in {1, i, -1, -i}; for the
-	 * component kept here (Re for even l + l1, Im for odd) the terms with p
-	 * of the other parity add +-0, so summing only p = l + l1 (mod 2), in
-	 * the same order, gives the same value bit for bit */
+	int K = L + 1, N = 2 * L + 1, Qp = (Q + SXS_QT - 1) / SXS_QT * SXS_QT;
+	int bx = blockIdx.x % nbx, zm = blockIdx.x / nbx;
+	int m = zm % K, iz = zm / K;
+	int j0 = m * K - m * (m - 1) / 2;         /* the pairs are in the order of l */
+	int t = bx * 128 + threadIdx.x;
+	if (t >= (nll1 - j0) * Qp) return;
+	int iq = t % Qp;
+	int2 pr = ll1[j0 + t / Qp];
+	int l = pr.x, l1 = pr.y;
 	double v = 0.0;
-	int p0 = l1 - l;  /* |l - l1| with l <= l1, same parity as l + l1 */
-	int odd = (l + l1) & 1;
-	for (int p = p0; p <= l + l1; p += 2) {
-		double w = sgn * dp[p] * bp[(size_t)p * Q];
-		/* i^p for even p: +1 (p % 4 == 0), -1 (p % 4 == 2); the imaginary unit
-		 * of i^p for odd p: +1 (p % 4 == 1), -1 (p % 4 == 3) */
-		int neg = odd ? ((p & 3) == 3) : ((p & 3) == 2);
-		v += (neg ? -1.0 : 1.0) * w;
+	if (iq < Q) {
+		const double *dp = ds + ((size_t)lm_index(l, m) * K + l1) * N;
+		const double *bp = bes + (size_t)iz * N * Q + iq;
+		int p0 = l1 - l;                      /* |l - l1| with l <= l1, same parity as l + l1 */
+		/* i^p: +1 (p % 4 == 0), -1 (2) for even p; the imaginary unit of i^p
+		 * for odd p: +1 (1), -1 (3); so the sign alternates with p */
+		bool neg = ((p0 & 2) != 0) != ((m & 1) != 0);
+		for (int p = p0; p <= l + l1; p += 2) {
+			double w = dp[p] * bp[(size_t)p * Q];
+			v = neg ? v - w : v + w;
+			neg = !neg;
+		}
 	}
 	/* q-tiled: [tile][iz][m][l][l1][SXS_QT], tile = q / SXS_QT */
 	size_t base = (((size_t)(iq / SXS_QT) * nz + iz) * K + m) * K;
-	tau[((base + l) * K + l1) * SXS_QT + iq % SXS_QT] = v;
-	tau[((base + l1) * K + l) * SXS_QT + iq % SXS_QT] = v;
+	double c28 = nu2 ? 268435456.0 / nu2[(size_t)iz * Qp + iq] : 0.0;
+	tau_store(tau + ((base + l) * K + l1) * SXS_QT + iq % SXS_QT, v, c28);
+	tau_store(tau + ((base + l1) * K + l) * SXS_QT + iq % SXS_QT, v, c28);
 }
 /* Cross terms of single molecules (src/min_saxs.c:450-494): for each
  * molecule and q, sum over lm of |V|^2, |D|^2, |W|^2, Re(V conj D),
@@ -638,27 +648,45 @@ __global__ void __launch_bounds__(128) k_sasa(const double *__restrict__ xyz, co
 	}
 }
 
+#define CI_CHUNK 256
+
 /* Self terms of fill_const (src/fftsaxs.c:27-50, 52-85): per channel pair
  * and q, sum over lm of Re(A1 conj A2) then Re(B1 conj B2), interleaved as in
- * comp_const_int, times {1,2,2,1,2,1}.  spf in the host flat layout. */
-__global__ void k_const_int(const double *__restrict__ A, const double *__restrict__ B, int Q, int L,
-                            double *__restrict__ cst)
+ * comp_const_int, times {1,2,2,1,2,1}.  spf in the host flat layout.  Block =
+ * (channel pair, q): all threads form the terms, one adds them in the
+ * reference's order.  0.043 ms at L = 20, Q = 101 (0.31 with a thread per sum
+ * that also read and multiplied, all of it latency), 0.16 at L = 30, Q = 201
+ * (0.67). */
+__global__ void __launch_bounds__(128) k_const_int(const double *__restrict__ A, const double *__restrict__ B, int Q,
+                                                   int L, double *__restrict__ cst)
 {
+	__shared__ double2 term[CI_CHUNK];
 	int K2 = (L + 1) * (L + 1);
-	int t = blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= 6 * Q) return;
-	int c = t / Q, iq = t % Q;
+	int c = blockIdx.x / Q, iq = blockIdx.x % Q;
 	const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 2};
 	const double mul[6] = {1.0, 2.0, 2.0, 1.0, 2.0, 1.0};
-	size_t chs = (size_t)Q * K2 * 2;
-	const double *a1 = A + pa[c] * chs + (size_t)iq * K2 * 2, *a2 = A + pb[c] * chs + (size_t)iq * K2 * 2;
-	const double *b1 = B + pa[c] * chs + (size_t)iq * K2 * 2, *b2 = B + pb[c] * chs + (size_t)iq * K2 * 2;
+	size_t chs = (size_t)Q * K2, at = (size_t)iq * K2;
+	const double2 *A2 = reinterpret_cast<const double2 *>(A), *B2 = reinterpret_cast<const double2 *>(B);
+	const double2 *a1 = A2 + pa[c] * chs + at, *a2 = A2 + pb[c] * chs + at;
+	const double2 *b1 = B2 + pa[c] * chs + at, *b2 = B2 + pb[c] * chs + at;
 	double s = 0.0;
-	for (int i = 0; i < K2; i++) {
-		s += a1[2 * i] * a2[2 * i] + a1[2 * i + 1] * a2[2 * i + 1];
-		s += b1[2 * i] * b2[2 * i] + b1[2 * i + 1] * b2[2 * i + 1];
+	for (int i0 = 0; i0 < K2; i0 += CI_CHUNK) {
+		int n = min(CI_CHUNK, K2 - i0);
+		for (int i = threadIdx.x; i < n; i += blockDim.x) {
+			double2 x = a1[i0 + i], y = a2[i0 + i], u = b1[i0 + i], v = b2[i0 + i];
+			term[i] = make_double2(x.x * y.x + x.y * y.y, u.x * v.x + u.y * v.y);
+		}
+		__syncthreads();
+		if (threadIdx.x == 0) {
+#pragma unroll 8
+			for (int i = 0; i < n; i++) {
+				s += term[i].x;
+				s += term[i].y;
+			}
+		}
+		__syncthreads();
 	}
-	cst[t] = s * mul[c];
+	if (threadIdx.x == 0) cst[c * Q + iq] = s * mul[c];
 }
 
 inline int nblk(long n, int b) { return (int)((n + b - 1) / b); }
@@ -696,9 +724,10 @@ int sxsk_expand_launches(void) { return 2; }
 
 int sxsk_bessel_z(const double *z, int nz, const double *q, int Q, int L, double *bes, cudaStream_t s)
 {
-	long n = (long)nz * Q * (2 * L + 1);
+	long n = (long)nz * Q, nb = (n + 127) / 128 * (2 * L + 1);
 	if (n == 0) return 0;
-	k_bessel_z<<<nblk(n, 128), 128, 0, s>>>(z, nz, q, Q, L, bes);
+	if (n > 0x7fffff00L || nb > 0x7fffffffL) return cudaErrorInvalidValue;
+	k_bessel_z<<<(unsigned)nb, 128, 0, s>>>(z, nz, q, Q, L, bes);
 	return cudaGetLastError();
 }
 
@@ -720,20 +749,24 @@ int sxsk_sasa(const double *xyz, const double *rad, int n, double probe, const d
 }
 
 int sxsk_tmatrix(const double *bes, const double *dsymb, int nz, int Q, int L, const int2 *ll1, int nll1,
-                 double *tau, cudaStream_t s)
+                 const double *nu2, void *tau, int form, cudaStream_t s)
 {
-	int K = L + 1;
-	long n = (long)nz * K * nll1 * Q;
-	if (n == 0) return 0;
-	size_t nt = (size_t)(Q + SXS_QT - 1) / SXS_QT;
-	cudaMemsetAsync(tau, 0, nt * nz * K * K * K * SXS_QT * sizeof(double), s);
-	k_tmatrix<<<nblk(n, 128), 128, 0, s>>>(bes, dsymb, nz, Q, L, ll1, nll1, tau);
+	int K = L + 1, Qp = (Q + SXS_QT - 1) / SXS_QT * SXS_QT;
+	long nbx = ((long)nll1 * Qp + 127) / 128, nb = nbx * nz * K;
+	if (nb == 0) return 0;
+	if (nb > 0x7fffffffL) return cudaErrorInvalidValue;
+	if (form == SXSK_TAU_FP32)
+		k_tmatrix<<<(unsigned)nb, 128, 0, s>>>(bes, dsymb, nz, Q, L, ll1, nll1, (int)nbx, nullptr, (float *)tau);
+	else if (form == SXSK_TAU_FIXED)
+		k_tmatrix<<<(unsigned)nb, 128, 0, s>>>(bes, dsymb, nz, Q, L, ll1, nll1, (int)nbx, nu2, (int2 *)tau);
+	else
+		k_tmatrix<<<(unsigned)nb, 128, 0, s>>>(bes, dsymb, nz, Q, L, ll1, nll1, (int)nbx, nullptr, (double *)tau);
 	return cudaGetLastError();
 }
 
 int sxsk_const_int(const double *A, const double *B, int Q, int L, double *cst, cudaStream_t s)
 {
-	k_const_int<<<nblk(6 * Q, 64), 64, 0, s>>>(A, B, Q, L, cst);
+	k_const_int<<<6 * Q, 128, 0, s>>>(A, B, Q, L, cst);
 	return cudaGetLastError();
 }
 

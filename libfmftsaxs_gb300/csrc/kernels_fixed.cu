@@ -25,6 +25,7 @@
  * the scale, and with it the result, NaN.
  */
 #include "kernels.h"
+#include "limbs.cuh"
 
 #include <math.h>
 
@@ -64,17 +65,6 @@ __device__ __forceinline__ int4 entry(i64 x, i64 y)
 {
 	int xh = hi_limb(x), yh = hi_limb(y);
 	return make_int4(xh, lo_limb(x, xh), yh, lo_limb(y, yh));
-}
-
-/* the limbs of v / 2^e, c28 = 2^(28 - e), |v| <= 2^(e + 1): a sum with 1.5 2^52
- * leaves the rounded integer in the low word, and the remainder is exact */
-__device__ __forceinline__ int2 limbs(double v, double c28)
-{
-	const double M = 6755399441055744.0;
-	double t = __fma_rn(v, c28, M);
-	double r = __fma_rn(v, c28, -__dsub_rn(t, M));
-	double u = __fma_rn(r, 536870912.0, M);
-	return make_int2(__double2loint(t), __double2loint(u));
 }
 
 /* sc[0][q] = 2^(28 - e), sc[1][q] = 2^e of a molecule's coefficients (host
@@ -131,14 +121,14 @@ __global__ void k_fix_spf(const double *__restrict__ flat, const double *__restr
 	long r = i / Q;
 	int lm = (int)(r % K2), ch = (int)(r / K2);
 	const double *s = flat + (((size_t)ch * Q + iq) * K2 + lm) * 2;
-	int2 a = limbs(s[0], sc[iq]), b = limbs(conj ? -s[1] : s[1], sc[iq]);
+	int2 a = sxs_limbs(s[0], sc[iq]), b = sxs_limbs(conj ? -s[1] : s[1], sc[iq]);
 	t[i] = make_int4(a.x, a.y, b.x, b.y);
 }
 
 __global__ void k_fix_dtab(const double *__restrict__ d, int2 *__restrict__ x, long n)
 {
 	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) x[i] = limbs(d[i], 268435456.0);
+	if (i < n) x[i] = sxs_limbs(d[i], 268435456.0);
 }
 
 /* nu2[iz][q] = 2^nu with |T(z q)|_2 <= 1.12 2^nu.  T is the compression to l
@@ -188,19 +178,6 @@ __global__ void __launch_bounds__(160) k_fix_nu(const double *__restrict__ bes, 
 	}
 }
 
-/* The translation matrices in place: tau [tile][iz][m][l][l1][8] (double) ->
- * limbs of tau / 2^nu */
-__global__ void k_fix_tau(double *__restrict__ tau, int nz, int K, int Qp, const double *__restrict__ nu2, long n)
-{
-	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	int q = (int)(i % SXS_QT);
-	long r = i / SXS_QT / ((long)K * K * K);
-	double s = nu2[(size_t)(r % nz) * Qp + (r / nz) * SXS_QT + q];
-	int2 v = limbs(tau[i], 268435456.0 / s);
-	reinterpret_cast<int2 *>(tau)[i] = v;
-}
-
 /* Twiddles of the paired rotation sum (kernels_contract.cu): h+ and h- as
  * limbs; of h+ = (tw[k] + tw[N-k]) / 2 the real part is the large one and of
  * h- = (tw[k] - tw[N-k]) / 2 the imaginary one.  The other parts vanish but
@@ -215,7 +192,7 @@ __device__ __forceinline__ FixTw fix_tw(const double2 *tw, int k, int N)
 {
 	int kk = k % N;
 	double2 a = tw[kk], b = tw[(N - kk) % N];
-	int2 c = limbs(0.5 * (a.x + b.x), 268435456.0), s = limbs(0.5 * (a.y - b.y), 268435456.0);
+	int2 c = sxs_limbs(0.5 * (a.x + b.x), 268435456.0), s = sxs_limbs(0.5 * (a.y - b.y), 268435456.0);
 	FixTw r;
 	r.a = make_int4(c.x, c.y, s.x, s.y);
 	r.b = make_int2((int)rint(0.5 * (a.y + b.y) * 0x1p57), (int)rint(0.5 * (a.x - b.x) * 0x1p57));
@@ -463,7 +440,7 @@ k_fix_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int 
 	__shared__ i64 F[12][FPC_THREADS];                /* the phased sums: six hh, six mid */
 	int K = L + 1, N = 2 * L + 1, NP = K * (K + 1) / 2, nrow = K * N;
 	for (int k = threadIdx.x; k < N; k += blockDim.x) {
-		int2 a = limbs(tw[k].x, 268435456.0), b = limbs(-tw[k].y, 268435456.0);
+		int2 a = sxs_limbs(tw[k].x, 268435456.0), b = sxs_limbs(-tw[k].y, 268435456.0);
 		tws[k] = make_int4(a.x, a.y, b.x, b.y);
 	}
 	__syncthreads();
@@ -593,14 +570,12 @@ int sxsk_fix_dtab(const double *d, int2 *x, long n, cudaStream_t s)
 	return cudaGetLastError();
 }
 
-int sxsk_fix_tau(const double *bes, double *tau, int nz, int Q, int L, double *nu2, cudaStream_t s)
+int sxsk_fix_nu(const double *bes, int nz, int Q, int L, double *nu2, cudaStream_t s)
 {
-	int NT = (Q + SXS_QT - 1) / SXS_QT, Qp = NT * SXS_QT, K = L + 1;
+	int Qp = (Q + SXS_QT - 1) / SXS_QT * SXS_QT;
 	if (nz <= 0) return 0;
-	long n = (long)NT * nz * K * K * K * SXS_QT;
-	if (L > SXSK_FIX_LMAX || (n + 255) / 256 > 0x7fffffffL || (long)nz * Qp > 0x7fffffffL) return cudaErrorInvalidValue;
+	if (L > SXSK_FIX_LMAX || (long)nz * Qp > 0x7fffffffL) return cudaErrorInvalidValue;
 	k_fix_nu<<<(unsigned)(nz * Qp), 160, 0, s>>>(bes, Q, L, Qp, nu2);
-	k_fix_tau<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(tau, nz, K, Qp, nu2, n);
 	return cudaGetLastError();
 }
 

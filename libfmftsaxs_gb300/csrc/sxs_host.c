@@ -241,8 +241,7 @@ struct sxsg_plan {
 	int nzt;                    /* touched z count */
 	double *h_zt, *d_zt;        /* touched z values */
 	double *d_bes;
-	double *d_tau;              /* [nzt][K][K][K][Q] */
-	float *d_tauf;              /* float copy (mixed path) */
+	void *d_tau;                /* [nzt][K][K][K][Q]: double or limbs, float on the mixed path */
 	/* per-chunk translated table */
 	void *d_R;
 	int64_t R_combos;
@@ -278,11 +277,11 @@ static void plan_free_poses(sxsg_plan *p)
 	pfree(p, p->d_slices);
 	p->h_slices = NULL; p->d_slices = NULL; p->nslice = 0;
 	pfree(p, p->d_poses); pfree(p, p->d_combo); pfree(p, p->d_zt); pfree(p, p->d_bes); pfree(p, p->d_tau);
-	pfree(p, p->d_tauf); pfree(p, p->d_cstart); pfree(p, p->d_nu2);
+	pfree(p, p->d_cstart); pfree(p, p->d_nu2);
 	p->d_cstart = NULL;
 	p->d_nu2 = NULL;
 	p->h_combo = NULL; p->h_cstart = NULL; p->h_zt = NULL;
-	p->d_poses = NULL; p->d_combo = NULL; p->d_zt = NULL; p->d_bes = NULL; p->d_tau = NULL; p->d_tauf = NULL;
+	p->d_poses = NULL; p->d_combo = NULL; p->d_zt = NULL; p->d_bes = NULL; p->d_tau = NULL;
 }
 
 void sxsg_plan_destroy(sxsg_plan *p)
@@ -649,8 +648,7 @@ int sxsg_plan_set_poses(sxsg_plan *p, const int64_t *index, int64_t n, int skip)
 	if (!e) e = cudaMallocAsync((void **)&p->d_zt, sizeof(double) * (nzt > 0 ? nzt : 1), p->s);
 	if (!e && nzt > 0) e = cudaMallocAsync((void **)&p->d_bes, sizeof(double) * (size_t)nzt * p->Q * N, p->s);
 	size_t tau_n = (size_t)p->NT * nzt * p->K * p->K * p->K * SXS_QT;
-	if (!e && nzt > 0) e = cudaMallocAsync((void **)&p->d_tau, sizeof(double) * tau_n, p->s);
-	if (!e && nzt > 0 && p->fp32) e = cudaMallocAsync((void **)&p->d_tauf, sizeof(float) * tau_n, p->s);
+	if (!e && nzt > 0) e = cudaMallocAsync(&p->d_tau, (p->fp32 ? sizeof(float) : sizeof(double)) * tau_n, p->s);
 	if (!e && ncombo > 0) e = cudaMemcpyAsync(p->d_combo, p->h_combo, sizeof(int32_t) * 3 * ncombo, cudaMemcpyHostToDevice, p->s);
 	if (!e) e = cudaMallocAsync((void **)&p->d_slices, sizeof(int32_t) * 2 * (p->nslice > 0 ? p->nslice : 1), p->s);
 	if (!e && p->nslice > 0)
@@ -685,22 +683,18 @@ int sxsg_plan_set_poses(sxsg_plan *p, const int64_t *index, int64_t n, int skip)
 	return 0;
 }
 
-/* per-z tables: Bessel values and translation matrices (FP64), in limbs for
- * a fixed-point run, with their float copy on the mixed path */
+/* per-z tables: Bessel values and translation matrices, computed in FP64 and
+ * written in the form that the run's translation reads */
 static int plan_ztables(sxsg_plan *p, cudaStream_t s)
 {
-	int L = p->L, Q = p->Q;
+	int L = p->L, Q = p->Q, form = p->fp32 ? SXSK_TAU_FP32 : (p->run_fixed ? SXSK_TAU_FIXED : SXSK_TAU_FP64);
 	SXS_K(sxsk_bessel_z(p->d_zt, p->nzt, p->d_q, Q, L, p->d_bes, s));
-	SXS_K(sxsk_tmatrix(p->d_bes, p->lt->d_dsymb, p->nzt, Q, L, p->lt->d_ll1, p->lt->nll1, p->d_tau, s));
-	sxs_count_launches(2);
-	if (p->run_fixed) {
-		SXS_K(sxsk_fix_tau(p->d_bes, p->d_tau, p->nzt, Q, L, p->d_nu2, s));
-		sxs_count_launches(2);
-	}
-	if (p->fp32) {
-		SXS_K(sxsk_to_float(p->d_tau, p->d_tauf, (long)p->NT * p->nzt * p->K * p->K * p->K * SXS_QT, s));
+	if (form == SXSK_TAU_FIXED) {
+		SXS_K(sxsk_fix_nu(p->d_bes, p->nzt, Q, L, p->d_nu2, s));
 		sxs_count_launches(1);
 	}
+	SXS_K(sxsk_tmatrix(p->d_bes, p->lt->d_dsymb, p->nzt, Q, L, p->lt->d_ll1, p->lt->nll1, p->d_nu2, p->d_tau, form, s));
+	sxs_count_launches(2);
 	return 0;
 }
 
@@ -821,7 +815,7 @@ int sxs_plan_batch_view(sxsg_plan *p, sxs_plan_view *v)
 	v->tr_slices = p->tr_slices; v->rot_gamma = p->rot_gamma; v->npose = p->npose;
 	v->fused = sxs_plan_uses_fused(p); v->cstart = p->d_cstart;
 	v->At = p->d_At; v->Bt = p->d_Bt; v->dtabf = p->lt->d_dtabf; v->tw = p->d_tw; v->P = p->d_P; v->U = p->d_U;
-	v->tauf = p->d_tauf; v->combo = p->d_combo; v->slices = p->d_slices; v->h_slices = p->h_slices;
+	v->tauf = p->d_tau; v->combo = p->d_combo; v->slices = p->d_slices; v->h_slices = p->h_slices;
 	v->h_cstart = p->h_cstart; v->poses = p->d_poses; v->cst = p->d_cstf; v->cross = p->d_cross;
 	v->fc = p->d_fc; v->c1g = p->d_c1g; v->c2g = p->d_c2g; v->gdf = p->d_gdf; v->a0sum = p->a0sum; v->peak = p->peak;
 	v->chi = p->d_chi; v->c1 = p->d_c1; v->c2 = p->d_c2; v->cell = p->d_cell;
@@ -961,7 +955,7 @@ int sxs_plan_enqueue(sxsg_plan *p, int fit_mode, int timed)
 	if (timed) SXS_CU(cudaEventRecord(p->ev[0], s));
 	if ((rc = plan_tables(p))) return rc;
 	if (timed) SXS_CU(cudaEventRecord(p->ev[1], s));
-	const void *tau = p->fp32 ? (const void *)p->d_tauf : (const void *)p->d_tau;
+	const void *tau = p->d_tau;
 	for (int64_t k = 0; k < nch; k++) {
 		int64_t s0 = p->h_chunk[k], s1 = p->h_chunk[k + 1];
 		int64_t c0 = p->h_slices[2 * s0], c1 = p->h_slices[2 * (s1 - 1)] + p->h_slices[2 * (s1 - 1) + 1];
@@ -1178,7 +1172,7 @@ size_t sxs_plan_base_bytes(int L, int Q, int nzt, int64_t npose, int n1, int pre
 	size_t spf = (size_t)3 * Q * K2;
 	size_t b = spf * (16 * 2 + celem * 2);                       /* A, B, At, Bt */
 	b += (size_t)nzt * Q * N * 8;                                /* Bessel */
-	b += NT * nzt * K * K * K * SXS_QT * (precision == SXSG_MIXED ? 12 : 8); /* tau */
+	b += NT * nzt * K * K * K * SXS_QT * (precision == SXSG_MIXED ? 4 : 8); /* tau */
 	b += (size_t)npose * (sizeof(sxsk_pose) + 6 * Q * 8 + 40);   /* poses, cross, outputs */
 	if (precision == SXSG_FP64) b += spf * 16 * 2 + (size_t)nzt * NT * SXS_QT * 8;   /* fixed-point inputs */
 	b += (size_t)n1 * Q * 16 + (size_t)64 * Q + (1 << 20);

@@ -234,6 +234,6 @@ def plan_bytes(L, Q, npose, nz):
     K, N, NT = L + 1, 2 * L + 1, (Q + 7) // 8
     NP = K * (K + 1) // 2
     rot = 2 * NT * K * N * NP * 3 * 8 * 8
-    tau = NT * nz * K ** 3 * 8 * 12 + nz * Q * N * 8
+    tau = NT * nz * K ** 3 * 8 * 4 + nz * Q * N * 8
     out = npose * (6 * Q * 8 + 4 * 8 + 8 + 32 + 8)
     return rot + tau + out + 64 * Q * K * K
