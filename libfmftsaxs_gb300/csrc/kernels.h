@@ -237,10 +237,13 @@ typedef struct {
 	int Q, L, conj, pad;
 } sxsk_rot_job;
 /* items {job, q tile, beta b, m}; G = gamma pairs per thread (the
- * single-dimer choice: 2, 4, 6, 8, 12 or 16); every job with N + (G-1) L
- * <= tw_max twiddle pairs */
-int sxsk_rotate_batch(const sxsk_rot_job *jobs, const int4 *items, int nitems, int G, int tw_max, int *ctr,
+ * single-dimer choice: 2, 4, 6, 8, 12 or 16); every job with L <= l_max and
+ * N + (G-1) L <= tw_max twiddle pairs */
+int sxsk_rotate_batch(const sxsk_rot_job *jobs, const int4 *items, int nitems, int G, int tw_max, int l_max, int *ctr,
                       cudaStream_t s);
+/* betas of one block of the FP32 rotation with G pairs per thread: the b of
+ * an item is the first of them, a multiple of this */
+int sxsk_rotate_betas(int G);
 
 typedef struct {
 	const void *U, *tau;              /* ligand rotation table, float tau of the job's z */

@@ -296,6 +296,116 @@ __device__ __forceinline__ void rotate_block(const typename Cx<S>::T *__restrict
 	}
 }
 
+/* The FP32 rotation from 8 gamma pairs per thread on (L >= 24).  Block = (m,
+ * two beta b0 and b0 + 1, q tile t); thread = (beta, group of G gamma pairs,
+ * channel, 2 adjacent q).  Per l the block forms S and D of every m1 once, in
+ * shared memory, for its four gamma groups (each group formed its own
+ * before, waiting for the coefficients: 2.8 of 6.7 stall cycles per
+ * instruction), and a twiddle load serves 8 multiply-adds instead of 4: the
+ * kernel is bound by shared-memory wavefronts, 24 per 64 multiply-adds of a
+ * warp (22 per 32 before).  2.73 -> 2.32 ms at L = 30, Q = 201 (staging 0.6,
+ * stores 0.1), 0.73 -> 0.61 at L = 25, Q = 101; six blocks per SM instead of
+ * the registers' five 2.50, seven 5.2 (spills).  The sums are those of
+ * rotate_block, bit for bit.  sd: the block's 2 L 24 staged entries. */
+#define ROT2_G 8
+#define ROT2_THREADS (2 * ROT_GROUPS * 3 * SXS_QP)
+#define ROT2_SMEM(L) (sizeof(float4) * 2 * (size_t)(L) * 3 * SXS_QT)
+template <int G>
+__device__ __forceinline__ void rotate2_block(const float2 *__restrict__ spf_t, const float *__restrict__ dtab,
+                                              const RotTw<float> *hs, float4 *sd, int Q, int L, int conj,
+                                              float2 *__restrict__ out, int t, int b0, int m)
+{
+	int K = L + 1, N = 2 * L + 1, K2 = K * K, NP = K * (K + 1) / 2, nrow = K * N;
+	float sg = conj ? -1.0f : 1.0f;
+	int sq = threadIdx.x % SXS_QT, sc = threadIdx.x / SXS_QT % 3, sr = threadIdx.x / (3 * SXS_QT);   /* staging */
+	int j2 = 2 * (threadIdx.x % SXS_QP), ch = threadIdx.x / SXS_QP % 3;
+	int gg = threadIdx.x / (3 * SXS_QP) % ROT_GROUPS, bb = threadIdx.x / (3 * SXS_QP * ROT_GROUPS);
+	int g0 = gg * G, b = b0 + bb;
+	bool act = b < K && g0 <= L, sok = t * SXS_QT + sq < Q;
+	const float *db = dtab + ((size_t)b0 * K * N + m + L) * N + L;   /* d^l_{m m1}(beta_b0) at l = 0, m1 = 0 */
+	size_t bstride = (size_t)K * N * N;                              /* between beta */
+	const float2 *Cs = spf_t + (size_t)sc * K2 * Q + (sok ? t * SXS_QT + sq : 0);
+	const float2 *C0 = spf_t + (size_t)ch * K2 * Q + t * SXS_QT + j2;
+	bool qa = t * SXS_QT + j2 < Q, qb = t * SXS_QT + j2 + 1 < Q;
+	float2 *ob = out + (((size_t)t * nrow + (size_t)b * N) * NP + psym(m, K)) * 3 * SXS_QT + ch * SXS_QT + j2;
+	size_t gstride = (size_t)NP * 3 * SXS_QT;
+	for (int l = m; l <= L; l++) {
+		const float *dl = db + (size_t)l * N * N;
+		const float2 *Cl = Cs + (size_t)l * (l + 1) * Q;             /* lm of m1 = 0 */
+		for (int r = sr; r < 2 * l; r += ROT2_THREADS / (3 * SXS_QT)) {
+			int ib = r >= l, m1 = r - (ib ? l : 0) + 1;
+			if (b0 + ib >= K) break;
+			float dp = __ldg(dl + ib * bstride + m1), dm = __ldg(dl + ib * bstride - m1);
+			float dps = mul_rn(dp, sg), dms = mul_rn(dm, sg);
+			float2 cp = zero2<float2>(), cm = zero2<float2>();
+			if (sok) {
+				cp = __ldg(Cl + (size_t)m1 * Q);
+				cm = __ldg(Cl - (ptrdiff_t)m1 * Q);
+			}
+			float mx = mul_rn(dm, cm.x), my = mul_rn(dms, cm.y);
+			sd[(r * 3 + sc) * SXS_QT + sq] = make_float4(fmaf(dp, cp.x, mx), fmaf(dps, cp.y, my), fmaf(dp, cp.x, -mx),
+			                                             fmaf(dps, cp.y, -my));
+		}
+		__syncthreads();
+		if (act) {
+			float d0 = __ldg(dl + bb * bstride), d0s = mul_rn(d0, sg);
+			const float2 *c0 = C0 + (size_t)l * (l + 1) * Q;
+			float2 ca = qa ? __ldg(c0) : zero2<float2>(), cb = qb ? __ldg(c0 + 1) : zero2<float2>();
+			float2 ya = make_float2(mul_rn(d0, ca.x), mul_rn(d0s, ca.y)), yb = make_float2(mul_rn(d0, cb.x), mul_rn(d0s, cb.y));
+			float2 Aa[G], Ba[G], Ab[G], Bb[G];
+#pragma unroll
+			for (int j = 0; j < G; j++) Aa[j] = Ba[j] = Ab[j] = Bb[j] = zero2<float2>();
+			int base = 0;                                        /* m1 g0 mod N */
+			const float4 *sp = sd + ((size_t)bb * l * 3 + ch) * SXS_QT + j2;
+			for (int m1 = 1; m1 <= l; m1++, sp += 3 * SXS_QT) {
+				base += g0;
+				if (base >= N) base -= N;
+				float4 va = sp[0], vb = sp[1];
+				float2 Sa = make_float2(va.x, va.y), Da = make_float2(va.z, va.w);
+				float2 Sb = make_float2(vb.x, vb.y), Db = make_float2(vb.z, vb.w);
+				int k = base;
+#pragma unroll
+				for (int j = 0; j < G; j++) {
+					RotTw<float> h = hs[k];
+					rot_acc(Aa[j], Ba[j], h, Sa, Da);
+					rot_acc(Ab[j], Bb[j], h, Sb, Db);
+					k += m1;
+				}
+			}
+			float2 *o = ob + (size_t)(l - m) * 3 * SXS_QT;
+#pragma unroll
+			for (int j = 0; j < G; j++) {
+				int g = g0 + j;
+				if (g > L) break;
+				float2 pa, ma, pb, mb;
+				rot_out(ya, Aa[j], Ba[j], pa, ma);
+				rot_out(yb, Ab[j], Bb[j], pb, mb);
+				st2(o + (size_t)g * gstride, pa, pb);
+				if (g > 0) st2(o + (size_t)(N - g) * gstride, ma, mb);
+			}
+		}
+		__syncthreads();
+	}
+}
+
+template <int G>
+__global__ void __launch_bounds__(ROT2_THREADS)
+k_rotate2(const float2 *__restrict__ spf_t, const float *__restrict__ dtab, const double2 *__restrict__ tw, int Q, int L,
+          int conj, float2 *__restrict__ out)
+{
+	extern __shared__ __align__(16) unsigned char rsm_raw[];
+	float4 *sd = reinterpret_cast<float4 *>(rsm_raw);
+	RotTw<float> *hs = reinterpret_cast<RotTw<float> *>(rsm_raw + ROT2_SMEM(L));   /* [N + (G-1) L] */
+	int K = L + 1, nb2 = (K + 1) / 2;
+	int bid = blockIdx.x;
+	int m = bid % K;
+	bid /= K;
+	int b0 = 2 * (bid % nb2), t = bid / nb2;
+	rotate_stage<float, G>(tw, L, hs);
+	__syncthreads();
+	rotate2_block<G>(spf_t, dtab, hs, sd, Q, L, conj, out, t, b0, m);
+}
+
 template <typename S, int G, int CH>
 __global__ void __launch_bounds__(ROT_THREADS(CH))
 k_rotate(const typename Cx<S>::T *__restrict__ spf_t, const S *__restrict__ dtab, const double2 *__restrict__ tw,
@@ -341,12 +451,13 @@ __device__ __forceinline__ int item_advance(int *ctr, int *s_it, int nxt, int ni
 
 /* rotation blocks of many tables (mixed path); the twiddles are restaged
  * when an item's table has other ones than the previous item's */
-template <int G, int CH>
-__global__ void __launch_bounds__(ROT_THREADS(CH))
-k_rotate_batch(const sxsk_rot_job *__restrict__ jobs, const int4 *__restrict__ items, int nitems, int *ctr)
+template <int G>
+__global__ void __launch_bounds__(G >= ROT2_G ? ROT2_THREADS : ROT_THREADS(3))
+k_rotate_batch(const sxsk_rot_job *__restrict__ jobs, const int4 *__restrict__ items, int nitems, int tw_max, int *ctr)
 {
 	extern __shared__ __align__(16) unsigned char rsm_raw[];
 	RotTw<float> *hs = reinterpret_cast<RotTw<float> *>(rsm_raw);
+	float4 *sd = reinterpret_cast<float4 *>(rsm_raw + (sizeof(RotTw<float>) * tw_max + 15) / 16 * 16);
 	const double2 *cur = nullptr;
 	int curL = -1;
 	__shared__ int s_it;
@@ -361,8 +472,12 @@ k_rotate_batch(const sxsk_rot_job *__restrict__ jobs, const int4 *__restrict__ i
 			cur = j.tw;
 			curL = j.L;
 		}
-		rotate_block<float, G, CH>((const float2 *)j.spf_t, (const float *)j.dtab, hs, j.Q, j.L, j.conj,
-		                           (float2 *)j.out, w.y, w.z, w.w);
+		if constexpr (G >= ROT2_G)
+			rotate2_block<G>((const float2 *)j.spf_t, (const float *)j.dtab, hs, sd, j.Q, j.L, j.conj, (float2 *)j.out, w.y,
+			                 w.z, w.w);
+		else
+			rotate_block<float, G, 3>((const float2 *)j.spf_t, (const float *)j.dtab, hs, j.Q, j.L, j.conj,
+			                          (float2 *)j.out, w.y, w.z, w.w);
 	}
 }
 
@@ -1437,12 +1552,12 @@ static int rotate_launch(const void *spf_t, const void *dtab, const double2 *tw,
                          cudaStream_t s)
 {
 	typedef typename Cx<S>::T V;
+	int K = L + 1, N = 2 * L + 1, NT = (Q + SXS_QT - 1) / SXS_QT;
 	/* three channels per thread in FP32 (one twiddle load for three) while
 	 * their 12 G accumulators leave room for warps (G <= 6, L <= 23: measured
-	 * 1.10 -> 1.04 ms at L = 20, slower from G = 8 on); FP64 is bound by its
-	 * arithmetic pipe and keeps one */
-	constexpr int CH = (sizeof(S) == 4 && G <= 6) ? 3 : 1;
-	int K = L + 1, N = 2 * L + 1, NT = (Q + SXS_QT - 1) / SXS_QT;
+	 * 1.10 -> 1.04 ms at L = 20); FP64 is bound by its arithmetic pipe and
+	 * keeps one */
+	constexpr int CH = sizeof(S) == 4 ? 3 : 1;
 	size_t smem = sizeof(RotTw<S>) * (size_t)(N + (G - 1) * L);
 	auto kern = k_rotate<S, G, CH>;
 	if (smem > 48 * 1024) {
@@ -1454,6 +1569,26 @@ static int rotate_launch(const void *spf_t, const void *dtab, const double2 *tw,
 	kern<<<(unsigned)nb, ROT_THREADS(CH), smem, s>>>((const V *)spf_t, (const S *)dtab, tw, Q, L, conj, (V *)out);
 	return cudaGetLastError();
 }
+
+template <int G>
+static int rotate2_launch(const void *spf_t, const void *dtab, const double2 *tw, int Q, int L, int conj, void *out,
+                          cudaStream_t s)
+{
+	int K = L + 1, N = 2 * L + 1, NT = (Q + SXS_QT - 1) / SXS_QT;
+	size_t smem = ROT2_SMEM(L) + sizeof(RotTw<float>) * (size_t)(N + (G - 1) * L);
+	auto kern = k_rotate2<G>;
+	if (smem > 48 * 1024) {
+		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		if (e != cudaSuccess) return e;
+	}
+	long nb = (long)K * ((K + 1) / 2) * NT;
+	if (nb > 0x7fffffffL) return cudaErrorInvalidValue;
+	kern<<<(unsigned)nb, ROT2_THREADS, smem, s>>>((const float2 *)spf_t, (const float *)dtab, tw, Q, L, conj,
+	                                              (float2 *)out);
+	return cudaGetLastError();
+}
+
+extern "C" int sxsk_rotate_betas(int G) { return G >= ROT2_G ? 2 : 1; }
 
 extern "C" int sxsk_rotate_group(int L, int gsel)
 {
@@ -1472,13 +1607,20 @@ static int rotate_any(const void *spf_t, const void *dtab, const double2 *tw, in
 	/* gamma pairs per thread: at least the L + 1 pairs over ROT_GROUPS
 	 * groups; a larger choice (gsel) leaves groups idle for fewer blocks'
 	 * worth of twiddle setup */
+	constexpr bool f32 = sizeof(S) == 4;
 	switch (sxsk_rotate_group(L, gsel)) {
 	case 2: return rotate_launch<S, 2>(spf_t, dtab, tw, Q, L, conj, out, s);
 	case 4: return rotate_launch<S, 4>(spf_t, dtab, tw, Q, L, conj, out, s);
 	case 6: return rotate_launch<S, 6>(spf_t, dtab, tw, Q, L, conj, out, s);
-	case 8: return rotate_launch<S, 8>(spf_t, dtab, tw, Q, L, conj, out, s);
-	case 12: return rotate_launch<S, 12>(spf_t, dtab, tw, Q, L, conj, out, s);
-	case 16: return rotate_launch<S, 16>(spf_t, dtab, tw, Q, L, conj, out, s);
+	case 8:
+		if constexpr (f32) return rotate2_launch<8>(spf_t, dtab, tw, Q, L, conj, out, s);
+		else return rotate_launch<S, 8>(spf_t, dtab, tw, Q, L, conj, out, s);
+	case 12:
+		if constexpr (f32) return rotate2_launch<12>(spf_t, dtab, tw, Q, L, conj, out, s);
+		else return rotate_launch<S, 12>(spf_t, dtab, tw, Q, L, conj, out, s);
+	case 16:
+		if constexpr (f32) return rotate2_launch<16>(spf_t, dtab, tw, Q, L, conj, out, s);
+		else return rotate_launch<S, 16>(spf_t, dtab, tw, Q, L, conj, out, s);
 	default: return cudaErrorInvalidValue;
 	}
 }
@@ -1505,18 +1647,19 @@ static cudaError_t persistent_grid(F kern, int threads, size_t smem, int nitems,
 }
 
 template <int G>
-static int rotate_batch_launch(const sxsk_rot_job *jobs, const int4 *items, int nitems, int tw_max, int *ctr,
+static int rotate_batch_launch(const sxsk_rot_job *jobs, const int4 *items, int nitems, int tw_max, int l_max, int *ctr,
                                cudaStream_t s)
 {
-	constexpr int CH = G <= 6 ? 3 : 1;   /* the FP32 choice of rotate_launch */
+	constexpr int threads = G >= ROT2_G ? ROT2_THREADS : ROT_THREADS(3);   /* the FP32 choice of rotate_launch */
 	size_t smem = sizeof(RotTw<float>) * (size_t)tw_max;
-	auto kern = k_rotate_batch<G, CH>;
+	if (G >= ROT2_G) smem = (smem + 15) / 16 * 16 + ROT2_SMEM(l_max);
+	auto kern = k_rotate_batch<G>;
 	cudaError_t e = cudaSuccess;
 	if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	int grid = 0;
-	if (!e) e = persistent_grid(kern, ROT_THREADS(CH), smem, nitems, ctr, &grid);
+	if (!e) e = persistent_grid(kern, threads, smem, nitems, ctr, &grid);
 	if (e) return e;
-	kern<<<grid, ROT_THREADS(CH), smem, s>>>(jobs, items, nitems, ctr);
+	kern<<<grid, threads, smem, s>>>(jobs, items, nitems, tw_max, ctr);
 	return cudaGetLastError();
 }
 
@@ -1740,17 +1883,17 @@ int sxsk_pose_cross(const sxsk_pose *poses, int npose, int combo_base, int ncomb
 	return cudaGetLastError();
 }
 
-int sxsk_rotate_batch(const sxsk_rot_job *jobs, const int4 *items, int nitems, int G, int tw_max, int *ctr,
+int sxsk_rotate_batch(const sxsk_rot_job *jobs, const int4 *items, int nitems, int G, int tw_max, int l_max, int *ctr,
                       cudaStream_t s)
 {
 	if (nitems <= 0) return 0;
 	switch (G) {
-	case 2: return rotate_batch_launch<2>(jobs, items, nitems, tw_max, ctr, s);
-	case 4: return rotate_batch_launch<4>(jobs, items, nitems, tw_max, ctr, s);
-	case 6: return rotate_batch_launch<6>(jobs, items, nitems, tw_max, ctr, s);
-	case 8: return rotate_batch_launch<8>(jobs, items, nitems, tw_max, ctr, s);
-	case 12: return rotate_batch_launch<12>(jobs, items, nitems, tw_max, ctr, s);
-	case 16: return rotate_batch_launch<16>(jobs, items, nitems, tw_max, ctr, s);
+	case 2: return rotate_batch_launch<2>(jobs, items, nitems, tw_max, l_max, ctr, s);
+	case 4: return rotate_batch_launch<4>(jobs, items, nitems, tw_max, l_max, ctr, s);
+	case 6: return rotate_batch_launch<6>(jobs, items, nitems, tw_max, l_max, ctr, s);
+	case 8: return rotate_batch_launch<8>(jobs, items, nitems, tw_max, l_max, ctr, s);
+	case 12: return rotate_batch_launch<12>(jobs, items, nitems, tw_max, l_max, ctr, s);
+	case 16: return rotate_batch_launch<16>(jobs, items, nitems, tw_max, l_max, ctr, s);
 	default: return cudaErrorInvalidValue;
 	}
 }

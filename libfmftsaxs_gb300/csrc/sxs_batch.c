@@ -244,13 +244,14 @@ static int build_rotations(sxsg_batch *b, bstage *st)
 	sxsk_rot_job *jobs = malloc(sizeof(sxsk_rot_job) * 2 * (size_t)b->n);
 	if (!jobs) return sxs_fail(-5, "out of host memory");
 	for (int gi = 0; gi < 6 && !rc; gi++) {
-		int G = gs[gi], nj = 0, twmax = 0;
+		int G = gs[gi], nj = 0, twmax = 0, lmax = 0, nbeta = sxsk_rotate_betas(G);
 		for (int i = 0; i < b->n && !rc; i++) {
 			const sxs_plan_view *v = &b->v[i];
 			if (sxsk_rotate_group(v->L, v->rot_gamma) != G) continue;
 			int K = v->L + 1, N = 2 * v->L + 1;
 			int tw = N + (G - 1) * v->L;
 			if (tw > twmax) twmax = tw;
+			if (v->L > lmax) lmax = v->L;
 			for (int tab = 0; tab < 2; tab++) {
 				sxsk_rot_job *j = &jobs[nj];
 				memset(j, 0, sizeof(*j));
@@ -263,17 +264,17 @@ static int build_rotations(sxsg_batch *b, bstage *st)
 				j->conj = tab;
 				size_t i0 = items.n;
 				for (int t = 0; t < v->NT && !rc; t++)
-					for (int bb = 0; bb < K && !rc; bb++)
+					for (int bb = 0; bb < K && !rc; bb += nbeta)
 						for (int m = 0; m < K && !rc; m++) {
 							/* multiply-adds of the block: sum over l >= m of l */
-							double cost = 0.5 * ((double)v->L * (v->L + 1) - (double)m * (m - 1)) + (K - m);
+							double cost = nbeta * 0.5 * ((double)v->L * (v->L + 1) - (double)m * (m - 1)) + nbeta * (K - m);
 							rc = add_item(&items, cost, nj, t, bb, m);
 						}
 				job_cost(&items, i0);
 				nj++;
 			}
 		}
-		if (!rc) rc = st_launch(st, 0, G | (twmax << 8), -1, jobs, sizeof(sxsk_rot_job) * nj, nj, &items, 0);
+		if (!rc) rc = st_launch(st, 0, G | (lmax << 8) | (twmax << 16), -1, jobs, sizeof(sxsk_rot_job) * nj, nj, &items, 0);
 	}
 	free(jobs);
 	free(items.p);
@@ -644,7 +645,7 @@ static int launch_one(sxsg_batch *b, const blaunch *L, int *ctr, const char *hba
 	if (!(b->flags & SXSG_BATCH_ITEMS) && (k == 1 || k == 2 || k == 4 || k == 5)) return launch_pieces(L, hbase, nk, s);
 	if (L->nitems > 0) (*nk)++;
 	switch (k) {
-	case 0: return sxsk_rotate_batch(jobs, items, L->nitems, L->arg & 0xff, L->arg >> 8, c, s);
+	case 0: return sxsk_rotate_batch(jobs, items, L->nitems, L->arg & 0xff, L->arg >> 16, (L->arg >> 8) & 0xff, c, s);
 	case 1: return sxsk_translate_batch(jobs, items, L->nitems, L->arg, c, s);
 	case 2: return sxsk_pose_cross_batch(jobs, items, L->nitems, c, s);
 	case 4: return sxsk_translate_fused_batch(jobs, items, L->nitems, L->arg, c, s);
