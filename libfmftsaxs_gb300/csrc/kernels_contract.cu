@@ -696,12 +696,24 @@ __device__ __forceinline__ void cp_async16(void *sdst, const void *gsrc)
 	unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
 	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
 }
+/* one float, zero when !in */
+__device__ __forceinline__ void cp_async4(float *sdst, const float *gsrc, bool in)
+{
+	unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gsrc), "r"(in ? 4 : 0) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
+/* float2 between the staged U columns of two combos: half a bank row more
+ * than the columns, because a half-warp reads 64 bytes of each of two combos
+ * (without it every such read took twice its wavefronts: 2.29 against 2.15
+ * ms at L = 20, Q = 101, all 18,000 combos) */
+#define TP_UROW(NB) ((NB) * 3 * SXS_QT + 8)
+
 /* shared bytes of k_translate_pipe<NB>: tau^m [8 q][NB NB + 4] and the U
  * columns of one slice [SXS_SLICE combos][NB pairs][3 ch][8 q] */
-#define TP_SMEM(NB) (sizeof(float) * SXS_QT * ((NB) * (NB) + 4) + sizeof(float2) * SXS_SLICE * (NB) * 3 * SXS_QT)
+#define TP_SMEM(NB) (sizeof(float) * SXS_QT * ((NB) * (NB) + 4) + sizeof(float2) * SXS_SLICE * TP_UROW(NB))
 
 /* The FP32 column form with three channels per thread, pipelined over
  * slices: block = (tile, run of sb consecutive slices, m); while the
@@ -710,9 +722,38 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
  * cp.async, so the global-load latency of the low occupancy that these
  * registers allow (1-5 blocks of 4 warps per SM by NB) overlaps the
  * arithmetic.  tau^m(q z) is restaged only where z changes between slices
- * (slices are z-major).  The sums are those of k_translate_col with CH = 3:
- * rows in even/odd pairs, one tau load for three channels. */
+ * (slices are z-major), by 4-byte cp.async as well, so that its one round
+ * trip to L2 overlaps the U columns'.  The sums are those of k_translate_col
+ * with CH = 3: rows in even/odd pairs, one tau load for three channels.
+ * A block's serial chain is what the low occupancy leaves visible: with the
+ * window of indices and tau through registers the above case took 2.02, now
+ * 1.96 ms (20,000 poses at L = 25: 3.22; 3.68 before the three changes). */
 #define TP_MINB(NB) (NB <= 8 ? 5 : (NB <= 12 ? 4 : (NB <= 20 ? 3 : (NB <= 28 ? 2 : 1))))
+
+/* The slices of a window of TP_W: first combo - cbase, combos, z; and per
+ * combo its row of U.  Read once per window by the whole block, so that the
+ * copies of a slice start without two dependent reads of global memory
+ * (2.15 -> 2.02 ms in the above case). */
+#define TP_W 8
+struct TpWin {
+	int4 sl[TP_W];
+	int row[TP_W][SXS_SLICE];
+};
+__device__ __forceinline__ void tp_window(TpWin &w, const int32_t *__restrict__ combo_zbg,
+                                          const int32_t *__restrict__ slices, int cbase, int s0, int s1, int N)
+{
+	__syncthreads();   /* no thread still reads the last window */
+	for (int i = threadIdx.x; i < TP_W * SXS_SLICE; i += TCOL_THREADS(3)) {
+		int s = s0 + i / SXS_SLICE, c = i % SXS_SLICE;
+		if (s >= s1) break;
+		int cf = slices[2 * s] - cbase, nc = slices[2 * s + 1];
+		if (c >= nc) continue;
+		const int32_t *z = combo_zbg + 3 * (cf + c);
+		w.row[i / SXS_SLICE][c] = z[1] * N + z[2];
+		if (c == 0) w.sl[i / SXS_SLICE] = make_int4(cf, nc, z[0], 0);
+	}
+	__syncthreads();
+}
 
 /* one block of k_translate_pipe: (tile t, slice group gi, m); raw = the
  * block's TP_SMEM(NB) bytes of shared memory */
@@ -732,13 +773,13 @@ __device__ __forceinline__ void tpipe_block(const float2 *__restrict__ U, const 
 	/* 16-byte chunks of one combo's n pairs: n x 3 x 8 float2 = 12 n; the
 	 * 8 threads of combo cl copy its chunks in 128-byte rows */
 	const int per = n * rowf / 2;
+	__shared__ TpWin win;
 	auto issue = [&](int s) {
-		int cf = slices[2 * s] - cbase, nc = slices[2 * s + 1];
-		if (cl < nc) {
-			int cc = cf + cl;
-			int b2 = combo_zbg[3 * cc + 1], g2 = combo_zbg[3 * cc + 2];
-			const float2 *src = U + (((size_t)t * nrow + b2 * N + g2) * NP + po) * rowf;
-			float2 *dst = us + (size_t)cl * NB * rowf;
+		if ((s - s0) % TP_W == 0) tp_window(win, combo_zbg, slices, cbase, s, s1, N);
+		int k = (s - s0) % TP_W;
+		if (cl < win.sl[k].y) {
+			const float2 *src = U + (((size_t)t * nrow + win.row[k][cl]) * NP + po) * rowf;
+			float2 *dst = us + (size_t)cl * TP_UROW(NB);
 			for (int r = q; r < per; r += SXS_QT) cp_async16(dst + 2 * r, src + 2 * r);
 		}
 		cp_async_commit();
@@ -746,18 +787,19 @@ __device__ __forceinline__ void tpipe_block(const float2 *__restrict__ U, const 
 	int zcur = -1;
 	if (s0 < s1) issue(s0);
 	for (int s = s0; s < s1; s++) {
-		int cf = slices[2 * s] - cbase, nc = slices[2 * s + 1];
-		int zi = combo_zbg[3 * cf];
+		int4 w = win.sl[(s - s0) % TP_W];
+		int cf = w.x, nc = w.y, zi = w.z;
 		if (zi != zcur) {
 			__syncthreads();   /* no thread still reads the previous tau */
 			const float *tz = tau + ((((size_t)t * nzt + zi) * K + m) * K) * K * SXS_QT;
-			for (int k = threadIdx.x; k < SXS_QT * NB * NB; k += blockDim.x) {
+			for (int k = threadIdx.x; k < SXS_QT * NB * NB; k += TCOL_THREADS(3)) {
 				int qq = k % SXS_QT, r = k / SXS_QT;
 				int i = r / NB, kk = r % NB;
-				float v = 0;
-				if (i < n && kk < n) v = __ldg(tz + ((size_t)(m + i) * K + m + kk) * SXS_QT + qq);
-				ts[qq * qstride + i * NB + kk] = v;
+				bool in = i < n && kk < n;
+				cp_async4(ts + qq * qstride + i * NB + kk,
+				          in ? tz + ((size_t)(m + i) * K + m + kk) * SXS_QT + qq : tz, in);
 			}
+			cp_async_commit();
 			zcur = zi;
 		}
 		cp_async_wait_all();
@@ -765,7 +807,7 @@ __device__ __forceinline__ void tpipe_block(const float2 *__restrict__ U, const 
 		bool act = cl < nc;
 		float2 u[3][NB];
 		if (act) {
-			const float2 *uc = us + (size_t)cl * NB * rowf + q;
+			const float2 *uc = us + (size_t)cl * TP_UROW(NB) + q;
 #pragma unroll
 			for (int j = 0; j < 3; j++)
 #pragma unroll
@@ -790,6 +832,159 @@ __device__ __forceinline__ void tpipe_block(const float2 *__restrict__ U, const 
 			}
 		}
 	}
+}
+
+/* The FP32 translation in tiles, for n = 29 to 32, whose 6 n registers of U
+ * leave the form above one block (a warp per scheduler) on an SM.  Block =
+ * (tile, run of sb consecutive slices, m), TT_CP combos at a time; thread =
+ * (q, two combos, TT_RB of the n rows).  Per k a thread reads TT_RB values
+ * tau[i][k] (kept transposed) and its combos' U[k] from shared memory for 96
+ * multiply-adds into 96 sums, each in the order of tcol_row.  82 KB and 219
+ * registers: two blocks.  L = 30, Q = 201, 40,000 poses, all classes: 18.5 ->
+ * 17.4 ms; for n = 25 to 28, where two blocks of the other form fit, it is
+ * the slower one (17.8), and so on down (19.3 with it everywhere). */
+#define TT_FROM 29
+#define TT_USE(NB) ((NB) >= TT_FROM)
+#define TT_RG 4
+#define TT_CP (32 / TT_RG)
+#define TT_RB(NB) ((((NB) + TT_RG - 1) / TT_RG + 1) / 2 * 2)
+#define TT_UROW(NB) ((NB) * 3 * SXS_QT + 4)   /* 4: see TP_UROW; a quarter-warp's combos are two rows apart */
+#define TT_TS(NB) ((NB) * TT_RB(NB) * TT_RG + 4)
+#define TT_SMEM(NB) (sizeof(float) * SXS_QT * TT_TS(NB) + sizeof(float2) * TT_CP * TT_UROW(NB))
+/* of the FP32 translation's blocks */
+#define TR_SMEM(NB) (TT_USE(NB) ? TT_SMEM(NB) : TP_SMEM(NB))
+#define TR_MINB(NB) (TT_USE(NB) ? 2 : TP_MINB(NB))
+
+template <int RB>
+struct TtIn {
+	float t[RB];
+	float2 u[2][3];
+};
+
+template <int NB>
+__device__ __forceinline__ void tt_load(TtIn<TT_RB(NB)> &x, const float *tq, const float2 *uq, int k)
+{
+	constexpr int RB = TT_RB(NB), RT = RB * TT_RG;
+	const float *t = tq + k * RT;
+	static_assert(RB % 4 == 0, "tau in 16-byte loads");
+#pragma unroll
+	for (int i = 0; i < RB / 4; i++) ld4(t + 4 * i, x.t + 4 * i);
+#pragma unroll
+	for (int c = 0; c < 2; c++)
+#pragma unroll
+		for (int j = 0; j < 3; j++) x.u[c][j] = uq[c * TT_UROW(NB) + (k * 3 + j) * SXS_QT];
+}
+
+template <int PK, int RB>
+__device__ __forceinline__ void tt_step(const TtIn<RB> &x, float2 (&acc)[2][3][RB])
+{
+#pragma unroll
+	for (int c = 0; c < 2; c++)
+#pragma unroll
+		for (int j = 0; j < 3; j++)
+#pragma unroll
+			for (int i = 0; i < RB; i++) {
+				float2 &a = acc[c][j][i];
+				float2 u = x.u[c][j];
+				if ((i & 1) == PK) {
+					a.x = fma_s(x.t[i], u.x, a.x);
+					a.y = fma_s(x.t[i], u.y, a.y);
+				} else {
+					a.x = fma_s(x.t[i], u.y, a.x);
+					a.y = fma_s(-x.t[i], u.x, a.y);
+				}
+			}
+}
+
+template <int NB>
+__device__ __forceinline__ void ttile_block(const float2 *__restrict__ U, const float *__restrict__ tau,
+                                            const int32_t *__restrict__ combo_zbg, const int32_t *__restrict__ slices,
+                                            int nslice, int cbase, int ncombo, int L, int nzt, int t, int gi, int m,
+                                            int sb, float2 *__restrict__ R, unsigned char *raw)
+{
+	constexpr int RB = TT_RB(NB), RT = RB * TT_RG, CP = TT_CP, rowf = 3 * SXS_QT;
+	constexpr int NTH = TCOL_THREADS(3), TPC = NTH / CP;   /* threads that copy a combo's columns */
+	float *ts = reinterpret_cast<float *>(raw);
+	float2 *us = reinterpret_cast<float2 *>(raw + sizeof(float) * SXS_QT * TT_TS(NB));
+	int K = L + 1, N = 2 * L + 1, NP = K * (K + 1) / 2, nrow = K * N;
+	int n = K - m, po = psym(m, K);
+	int s0 = gi * sb, s1 = s0 + sb < nslice ? s0 + sb : nslice;
+	int tid = threadIdx.x, q = tid % SXS_QT, pr = tid / SXS_QT % (CP / 2), i0 = tid / (SXS_QT * (CP / 2)) * RB;
+	__shared__ TpWin win;
+	int zcur = -1;
+	for (int s = s0; s < s1; s++) {
+		if ((s - s0) % TP_W == 0) tp_window(win, combo_zbg, slices, cbase, s, s1, N);
+		int4 w = win.sl[(s - s0) % TP_W];
+		int cf = w.x, nc = w.y, zi = w.z;
+		for (int h = 0; h < nc; h += CP) {
+			int nh = min(CP, nc - h);
+			__syncthreads();   /* no thread still reads tau or U */
+			int cl = tid / TPC;
+			if (cl < nh) {
+				const float2 *src = U + (((size_t)t * nrow + win.row[(s - s0) % TP_W][h + cl]) * NP + po) * rowf;
+				float2 *dst = us + (size_t)cl * TT_UROW(NB);
+				for (int r = tid % TPC; r < n * rowf / 2; r += TPC) cp_async16(dst + 2 * r, src + 2 * r);
+			}
+			cp_async_commit();
+			if (zi != zcur) {
+				const float *tz = tau + ((((size_t)t * nzt + zi) * K + m) * K) * K * SXS_QT;
+				for (int k = tid; k < SXS_QT * NB * RT; k += NTH) {
+					int qq = k % SXS_QT, r = k / SXS_QT;
+					int i = r % RT, kk = r / RT;
+					bool in = i < n && kk < n;
+					cp_async4(ts + qq * TT_TS(NB) + kk * RT + i,
+					          in ? tz + ((size_t)(m + i) * K + m + kk) * SXS_QT + qq : tz, in);
+				}
+				cp_async_commit();
+				zcur = zi;
+			}
+			cp_async_wait_all();
+			__syncthreads();   /* these U columns and tau visible to all */
+			if (2 * pr >= nh || i0 >= n) continue;
+			const float *tq = ts + q * TT_TS(NB) + i0;
+			const float2 *uq = us + (size_t)2 * pr * TT_UROW(NB) + q;
+			float2 acc[2][3][RB];
+#pragma unroll
+			for (int c = 0; c < 2; c++)
+#pragma unroll
+				for (int j = 0; j < 3; j++)
+#pragma unroll
+					for (int i = 0; i < RB; i++) acc[c][j][i] = make_float2(0.0f, 0.0f);
+			TtIn<RB> x, y;
+			tt_load<NB>(x, tq, uq, 0);
+			int k = 0;
+			for (; k + 1 < n; k += 2) {
+				tt_load<NB>(y, tq, uq, k + 1);
+				tt_step<0>(x, acc);
+				tt_load<NB>(x, tq, uq, min(k + 2, n - 1));
+				tt_step<1>(y, acc);
+			}
+			if (k < n) tt_step<0>(x, acc);
+#pragma unroll
+			for (int c = 0; c < 2; c++) {
+				if (2 * pr + c >= nh) break;
+				float2 *Rb = R + (((size_t)t * ncombo + cf + h + 2 * pr + c) * NP + po + i0) * rowf + q;
+#pragma unroll
+				for (int i = 0; i < RB; i++)
+					if (i0 + i < n)
+#pragma unroll
+						for (int j = 0; j < 3; j++) Rb[(size_t)i * rowf + j * SXS_QT] = acc[c][j][i];
+			}
+		}
+	}
+}
+
+template <int NB>
+__device__ __forceinline__ void translate_block(const float2 *__restrict__ U, const float *__restrict__ tau,
+                                                const int32_t *__restrict__ combo_zbg,
+                                                const int32_t *__restrict__ slices, int nslice, int cbase, int ncombo,
+                                                int L, int nzt, int t, int gi, int m, int sb, float2 *__restrict__ R,
+                                                unsigned char *raw)
+{
+	if constexpr (TT_USE(NB))
+		ttile_block<NB>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, L, nzt, t, gi, m, sb, R, raw);
+	else
+		tpipe_block<NB>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, L, nzt, t, gi, m, sb, R, raw);
 }
 
 /* poses per pass of a thread of the fused kernel: the per-pose sums
@@ -858,7 +1053,7 @@ __device__ __forceinline__ void tfused_block(const float2 *__restrict__ U, const
 			int cc = cf + cl;
 			int b2 = combo_zbg[3 * cc + 1], g2 = combo_zbg[3 * cc + 2];
 			const float2 *src = U + (((size_t)t * nrow + b2 * N + g2) * NP + po) * rowf;
-			float2 *dst = us + (size_t)cl * NB * rowf;
+			float2 *dst = us + (size_t)cl * TP_UROW(NB);
 			for (int r = q; r < per; r += SXS_QT) cp_async16(dst + 2 * r, src + 2 * r);
 		}
 		cp_async_commit();
@@ -885,7 +1080,7 @@ __device__ __forceinline__ void tfused_block(const float2 *__restrict__ U, const
 		bool act = cl < nc;
 		float2 u[3][NB];
 		if (act) {
-			const float2 *uc = us + (size_t)cl * NB * rowf + q;
+			const float2 *uc = us + (size_t)cl * TP_UROW(NB) + q;
 #pragma unroll
 			for (int j = 0; j < 3; j++)
 #pragma unroll
@@ -974,7 +1169,7 @@ k_translate_fused_batch(const sxsk_tf_job *__restrict__ jobs, const int4 *__rest
 }
 
 template <int NB>
-__global__ void __launch_bounds__(TCOL_THREADS(3), TP_MINB(NB))
+__global__ void __launch_bounds__(TCOL_THREADS(3), TR_MINB(NB))
 k_translate_pipe(const float2 *__restrict__ U, const float *__restrict__ tau, const int32_t *__restrict__ combo_zbg,
                  const int32_t *__restrict__ slices, int nslice, int cbase, int ncombo, int L, int nzt, int m_lo,
                  int nm, int sb, float2 *__restrict__ R)
@@ -985,12 +1180,12 @@ k_translate_pipe(const float2 *__restrict__ U, const float *__restrict__ tau, co
 	int mi = bid % nm;
 	bid /= nm;
 	int gi = bid % ng, t = bid / ng;
-	tpipe_block<NB>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, L, nzt, t, gi, m_lo + mi, sb, R, tps_raw);
+	translate_block<NB>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, L, nzt, t, gi, m_lo + mi, sb, R, tps_raw);
 }
 
 /* pipelined translation blocks of many chunks (mixed path) */
 template <int NB>
-__global__ void __launch_bounds__(TCOL_THREADS(3), TP_MINB(NB))
+__global__ void __launch_bounds__(TCOL_THREADS(3), TR_MINB(NB))
 k_translate_batch(const sxsk_tr_job *__restrict__ jobs, const int4 *__restrict__ items, int nitems, int *ctr)
 {
 	extern __shared__ __align__(16) unsigned char tps_raw[];
@@ -1000,7 +1195,7 @@ k_translate_batch(const sxsk_tr_job *__restrict__ jobs, const int4 *__restrict__
 		nxt = item_claim(ctr);
 		int4 w = items[it];
 		sxsk_tr_job j = jobs[w.x];
-		tpipe_block<NB>((const float2 *)j.U, (const float *)j.tau, j.combo_zbg, j.slices, j.nslice, j.cbase,
+		translate_block<NB>((const float2 *)j.U, (const float *)j.tau, j.combo_zbg, j.slices, j.nslice, j.cbase,
 		                j.ncombo, j.L, j.nzt, w.y, w.z, w.w, j.sb, (float2 *)j.R, tps_raw);
 	}
 }
@@ -1469,7 +1664,7 @@ static cudaError_t translate_col_launch(const void *U, const void *tau, const in
 		/* FP32: three channels per thread, pipelined over runs of slices */
 		long nb = (long)NT * ((nslice + sb - 1) / sb) * nm;
 		if (nb > 0x7fffffffL) return cudaErrorInvalidValue;
-		size_t smem = TP_SMEM(NB);
+		size_t smem = TR_SMEM(NB);
 		auto kern = k_translate_pipe<NB>;
 		if (smem > 48 * 1024) {
 			cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1666,7 +1861,7 @@ static int rotate_batch_launch(const sxsk_rot_job *jobs, const int4 *items, int 
 template <int NB>
 static int translate_batch_launch(const sxsk_tr_job *jobs, const int4 *items, int nitems, int *ctr, cudaStream_t s)
 {
-	size_t smem = TP_SMEM(NB);
+	size_t smem = TR_SMEM(NB);
 	auto kern = k_translate_batch<NB>;
 	cudaError_t e = cudaSuccess;
 	if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
