@@ -135,9 +135,12 @@ int sxsk_rotate_group(int L, int gsel);
 /* slices per block of the pipelined FP32 translation when a plan sets none */
 #define SXSK_TP_SB 8
 /* the launch of sxsk_translate (FP32) for column class NB alone (the m with
- * L + 1 - m in (NB - 4, NB]); nothing when the class has no m for L */
+ * L + 1 - m in (NB - 4, NB]); nothing when the class has no m for L.
+ * linked: the stream's last launch is another of these, for other rows, and
+ * this one need not wait for it (chain.cuh) */
 int sxsk_translate_class(const void *U, const void *tau, const int32_t *combo_zbg, const int32_t *slices, int nslice,
-                         int cbase, int ncombo, int nzt, int Q, int L, void *R, int sb, int NB, cudaStream_t s);
+                         int cbase, int ncombo, int nzt, int Q, int L, void *R, int sb, int NB, int linked,
+                         cudaStream_t s);
 /* kernel launches one sxsk_translate call makes for this L */
 int sxsk_translate_launches(int L);
 /* translated ligand table for the combos of a run of slices, m >= 0, all q tiles:

@@ -22,6 +22,7 @@
  * tabulated: pairs (m, l), m = 0..L, l = m..L, (L+1)(L+2)/2 of them.
  */
 #include "kernels.h"
+#include "chain.cuh"
 
 namespace {
 
@@ -1175,12 +1176,14 @@ k_translate_pipe(const float2 *__restrict__ U, const float *__restrict__ tau, co
                  int nm, int sb, float2 *__restrict__ R)
 {
 	extern __shared__ __align__(16) unsigned char tps_raw[];
+	chain_begin();
 	int ng = (nslice + sb - 1) / sb;
 	int bid = blockIdx.x;
 	int mi = bid % nm;
 	bid /= nm;
 	int gi = bid % ng, t = bid / ng;
 	translate_block<NB>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, L, nzt, t, gi, m_lo + mi, sb, R, tps_raw);
+	chain_end();
 }
 
 /* pipelined translation blocks of many chunks (mixed path) */
@@ -1650,7 +1653,7 @@ inline int nblk(long n, int b) { return (int)((n + b - 1) / b); }
 template <typename S, int NB>
 static cudaError_t translate_col_launch(const void *U, const void *tau, const int32_t *combo_zbg,
                                         const int32_t *slices, int nslice, int cbase, int ncombo, int nzt, int NT,
-                                        int L, void *R, int sb, cudaStream_t s)
+                                        int L, void *R, int sb, bool *linked, cudaStream_t s)
 {
 	typedef typename Cx<S>::T V;
 	int K = L + 1;
@@ -1674,9 +1677,10 @@ static cudaError_t translate_col_launch(const void *U, const void *tau, const in
 		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
 		                                     (int)cudaSharedmemCarveoutMaxShared);
 		if (e != cudaSuccess) return e;
-		kern<<<(unsigned)nb, TCOL_THREADS(3), smem, s>>>((const float2 *)U, (const float *)tau, combo_zbg, slices,
-		                                                 nslice, cbase, ncombo, L, nzt, m_lo, nm, sb, (float2 *)R);
-		return cudaGetLastError();
+		e = chain_launch(kern, (unsigned)nb, TCOL_THREADS(3), smem, s, *linked, (const float2 *)U, (const float *)tau,
+		                 combo_zbg, slices, nslice, cbase, ncombo, L, nzt, m_lo, nm, sb, (float2 *)R);
+		*linked = true;
+		return e;
 	} else {
 		/* FP64 (bound by its pipe): one channel per thread */
 		long nb = (long)NT * nslice * nm;
@@ -1699,14 +1703,15 @@ static cudaError_t translate_col_all(const void *U, const void *tau, const int32
                                      cudaStream_t s)
 {
 	cudaError_t e = cudaSuccess;
-	if (!e) e = translate_col_launch<S, 4>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
-	if (!e) e = translate_col_launch<S, 8>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
-	if (!e) e = translate_col_launch<S, 12>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
-	if (!e) e = translate_col_launch<S, 16>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
-	if (!e) e = translate_col_launch<S, 20>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
-	if (!e) e = translate_col_launch<S, 24>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
-	if (!e) e = translate_col_launch<S, 28>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
-	if (!e) e = translate_col_launch<S, 32>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
+	bool linked = false;
+	if (!e) e = translate_col_launch<S, 4>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
+	if (!e) e = translate_col_launch<S, 8>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
+	if (!e) e = translate_col_launch<S, 12>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
+	if (!e) e = translate_col_launch<S, 16>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
+	if (!e) e = translate_col_launch<S, 20>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
+	if (!e) e = translate_col_launch<S, 24>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
+	if (!e) e = translate_col_launch<S, 28>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
+	if (!e) e = translate_col_launch<S, 32>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, &linked, s);
 	return e;
 }
 
@@ -1959,14 +1964,17 @@ int sxsk_pose_scatter(const sxsk_pose *tmp, const int32_t *key, int64_t n, int32
 }
 
 int sxsk_translate_class(const void *U, const void *tau, const int32_t *combo_zbg, const int32_t *slices, int nslice,
-                         int cbase, int ncombo, int nzt, int Q, int L, void *R, int sb, int NB, cudaStream_t s)
+                         int cbase, int ncombo, int nzt, int Q, int L, void *R, int sb, int NB, int linked, cudaStream_t s)
 {
 	if (nslice <= 0) return 0;
 	if (L + 1 > 32) return cudaErrorInvalidValue;
 	int NT = (Q + SXS_QT - 1) / SXS_QT;
 	if (sb < 1) sb = SXSK_TP_SB;
+	bool lk = linked;
 #define TCL(C)                                                                                                     \
-	case C: return translate_col_launch<float, C>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb, s);
+	case C:                                                                                                        \
+		return translate_col_launch<float, C>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, sb,  \
+		                                      &lk, s);
 	switch (NB) {
 		TCL(4) TCL(8) TCL(12) TCL(16) TCL(20) TCL(24) TCL(28) TCL(32)
 	default: return cudaErrorInvalidValue;

@@ -25,6 +25,7 @@
  * the scale, and with it the result, NaN.
  */
 #include "kernels.h"
+#include "chain.cuh"
 #include "limbs.cuh"
 
 #include <math.h>
@@ -341,6 +342,7 @@ k_fix_translate(const int4 *__restrict__ U, const int2 *__restrict__ tau, const 
                 int4 *__restrict__ R)
 {
 	extern __shared__ __align__(16) unsigned char ftsm[];
+	chain_begin();
 	int2 *ts = reinterpret_cast<int2 *>(ftsm);   /* [8 q][NB i][NB k] (+ pad per q) */
 	const int qstride = NB * NB + 2;
 	int K = L + 1, N = 2 * L + 1, NP = K * (K + 1) / 2, nrow = K * N;
@@ -353,7 +355,10 @@ k_fix_translate(const int4 *__restrict__ U, const int2 *__restrict__ tau, const 
 	int si = bid % nslice, t = bid / nslice;
 	int m = m_lo + mi, n = K - m;
 	int cfirst = slices[2 * si] - cbase + part * FTR_COMBOS, nc = slices[2 * si + 1] - part * FTR_COMBOS;
-	if (nc <= 0) return;
+	if (nc <= 0) {
+		chain_end();
+		return;
+	}
 	int zi = combo_zbg[3 * cfirst];
 	const int2 *tz = tau + ((((size_t)t * nzt + zi) * K + m) * K) * K * SXS_QT;
 	for (int k = threadIdx.x; k < SXS_QT * NB * NB; k += blockDim.x) {
@@ -372,13 +377,15 @@ k_fix_translate(const int4 *__restrict__ U, const int2 *__restrict__ tau, const 
 #pragma unroll
 	for (int k = 0; k < NB; k++) u[k] = k < n ? __ldg(Ub + (size_t)k * 3 * SXS_QT) : make_int4(0, 0, 0, 0);
 	__syncthreads();
-	if (!act) return;
-	const int2 *tq = ts + q * qstride;
-	int4 *Rb = R + (((size_t)t * ncombo + c) * NP + po) * 3 * SXS_QT + ch * SXS_QT + q;
-	for (int i = 0; i < n; i += 2) {
-		Rb[(size_t)i * 3 * SXS_QT] = fix_row<0, NB>(tq + i * NB, u);
-		if (i + 1 < n) Rb[(size_t)(i + 1) * 3 * SXS_QT] = fix_row<1, NB>(tq + (i + 1) * NB, u);
+	if (act) {
+		const int2 *tq = ts + q * qstride;
+		int4 *Rb = R + (((size_t)t * ncombo + c) * NP + po) * 3 * SXS_QT + ch * SXS_QT + q;
+		for (int i = 0; i < n; i += 2) {
+			Rb[(size_t)i * 3 * SXS_QT] = fix_row<0, NB>(tq + i * NB, u);
+			if (i + 1 < n) Rb[(size_t)(i + 1) * 3 * SXS_QT] = fix_row<1, NB>(tq + (i + 1) * NB, u);
+		}
 	}
+	chain_end();
 }
 
 /* 16-byte loads with L2 policies: receptor rows are read by many poses
@@ -528,7 +535,7 @@ int rotate_launch(const void *spf, const int2 *dtab, const double2 *tw, int Q, i
 
 template <int NB>
 int translate_launch(const void *U, const void *tau, const int32_t *combo_zbg, const int32_t *slices, int nslice,
-                     int cbase, int ncombo, int nzt, int NT, int L, void *R, cudaStream_t s)
+                     int cbase, int ncombo, int nzt, int NT, int L, void *R, bool *linked, cudaStream_t s)
 {
 	int K = L + 1;
 	/* m with n = K - m in (NB - 4, NB] */
@@ -547,9 +554,10 @@ int translate_launch(const void *U, const void *tau, const int32_t *combo_zbg, c
 		e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
 		                         (int)cudaSharedmemCarveoutMaxShared);
 	if (e) return e;
-	kern<<<(unsigned)nb, FTR_THREADS, smem, s>>>((const int4 *)U, (const int2 *)tau, combo_zbg, slices, nslice, cbase,
-	                                             ncombo, L, nzt, m_lo, nm, (int4 *)R);
-	return cudaGetLastError();
+	e = chain_launch(kern, (unsigned)nb, FTR_THREADS, smem, s, *linked, (const int4 *)U, (const int2 *)tau, combo_zbg,
+	                 slices, nslice, cbase, ncombo, L, nzt, m_lo, nm, (int4 *)R);
+	*linked = true;
+	return e;
 }
 
 } // namespace
@@ -598,8 +606,9 @@ int sxsk_fix_translate(const void *U, const void *tau, const int32_t *combo_zbg,
 	if (nslice <= 0) return 0;
 	if (L > SXSK_FIX_LMAX) return cudaErrorInvalidValue;
 	int NT = (Q + SXS_QT - 1) / SXS_QT, e = 0;
+	bool linked = false;
 #define FTL(NB) \
-	if (!e) e = translate_launch<NB>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, s);
+	if (!e) e = translate_launch<NB>(U, tau, combo_zbg, slices, nslice, cbase, ncombo, nzt, NT, L, R, &linked, s);
 	FTL(4) FTL(8) FTL(12) FTL(16) FTL(20) FTL(24) FTL(28) FTL(32)
 #undef FTL
 	return e;

@@ -606,17 +606,19 @@ static int class_used(int L, int NB)
 
 /* The translation and per-pose launches of a phase without work items: the
  * single-dimer kernels, one launch per piece (and column class), read from
- * the host copy of the jobs.  *nk += the kernels launched. */
+ * the host copy of the jobs.  The pieces of one call do not depend on one
+ * another and form a chain (chain.cuh).  *nk += the kernels launched. */
 static int launch_pieces(const blaunch *L, const char *hbase, int *nk, cudaStream_t s)
 {
 	const char *hj = hbase + L->jobs_off;
-	int rc = 0;
+	int rc = 0, linked = 0;
 	for (int j = 0; j < L->njobs && !rc; j++) {
 		if (L->kind == 1) {
 			const sxsk_tr_job *t = (const sxsk_tr_job *)hj + j;
 			if (!class_used(t->L, L->arg)) continue;
 			rc = sxsk_translate_class(t->U, t->tau, t->combo_zbg, t->slices, t->nslice, t->cbase, t->ncombo, t->nzt,
-			                          t->Q, t->L, t->R, t->sb, L->arg, s);
+			                          t->Q, t->L, t->R, t->sb, L->arg, linked, s);
+			linked |= t->nslice > 0;
 		} else if (L->kind == 4) {
 			const sxsk_tf_job *t = (const sxsk_tf_job *)hj + j;
 			if (!class_used(t->L, L->arg)) continue;
