@@ -156,9 +156,11 @@ int sxsk_translate(const void *U, const void *tau, const int32_t *combo_zbg, con
  * the m < 0 half folded in by symmetry; R holds the ncombo combos from combo_base.
  * FP64 path: cst and cross are double.  FP32 path: cst and cross are
  * double-float pairs {hi, lo} (float2), so that neither this kernel nor the
- * fit that reads the terms touches the FP64 pipe. */
+ * fit that reads the terms touches the FP64 pipe.  linked: as above, for
+ * other poses; -1: the launch is not one of several. */
 int sxsk_pose_cross(const sxsk_pose *poses, int npose, int combo_base, int ncombo, const void *P, const void *R,
-                    const double2 *tw, const void *cst, int Q, int L, void *cross, int fp32, cudaStream_t s);
+                    const double2 *tw, const void *cst, int Q, int L, void *cross, int fp32, int linked,
+                    cudaStream_t s);
 /* The mixed path's translation fused with the per-pose contraction, for
  * sparse pose lists (few poses per translated row): the translated rows of
  * the chunk's combos are never stored; per pose and m the six channel sums

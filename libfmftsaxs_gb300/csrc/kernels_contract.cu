@@ -1381,11 +1381,11 @@ __device__ __forceinline__ void pcross_block(const sxsk_pose *__restrict__ poses
 }
 
 template <typename S, bool HINT>
-__global__ void __launch_bounds__(128)
-k_pose_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int ncombo,
-             const typename Cx<S>::T *__restrict__ P, const typename Cx<S>::T *__restrict__ R,
-             const double2 *__restrict__ tw, const typename CrossT<S>::T *__restrict__ cst, int Q, int L,
-             typename CrossT<S>::T *__restrict__ cross)
+__device__ __forceinline__ void pcross_grid(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int ncombo,
+                                            const typename Cx<S>::T *__restrict__ P,
+                                            const typename Cx<S>::T *__restrict__ R, const double2 *__restrict__ tw,
+                                            const typename CrossT<S>::T *__restrict__ cst, int Q, int L,
+                                            typename CrossT<S>::T *__restrict__ cross)
 {
 	typedef typename Cx<S>::T V;
 	__shared__ V tws[2 * SXS_LMAX_K - 1];
@@ -1395,6 +1395,31 @@ k_pose_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int
 	int bpt = (npose + PC_PPB - 1) / PC_PPB;
 	int t = blockIdx.x / bpt, pb = blockIdx.x % bpt;
 	pcross_block<S, HINT>(poses, npose, combo_base, ncombo, P, R, tws, cst, Q, L, cross, t, pb);
+}
+
+template <typename S, bool HINT>
+__global__ void __launch_bounds__(128)
+k_pose_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int ncombo,
+             const typename Cx<S>::T *__restrict__ P, const typename Cx<S>::T *__restrict__ R,
+             const double2 *__restrict__ tw, const typename CrossT<S>::T *__restrict__ cst, int Q, int L,
+             typename CrossT<S>::T *__restrict__ cross)
+{
+	pcross_grid<S, HINT>(poses, npose, combo_base, ncombo, P, R, tw, cst, Q, L, cross);
+}
+
+/* The same with the loads of two pairs in flight: 93 registers and POSE_DEEP
+ * blocks on an SM instead of 56 and POSE_FLAT.  Faster where rows come from
+ * DRAM (pose_deep below). */
+#define POSE_FLAT 9
+#define POSE_DEEP 5
+__global__ void __launch_bounds__(128, POSE_DEEP)
+k_pose_cross_deep(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int ncombo,
+                  const float2 *__restrict__ P, const float2 *__restrict__ R, const double2 *__restrict__ tw,
+                  const float2 *__restrict__ cst, int Q, int L, float2 *__restrict__ cross)
+{
+	chain_begin();
+	pcross_grid<float, true>(poses, npose, combo_base, ncombo, P, R, tw, cst, Q, L, cross);
+	chain_end();
 }
 
 /* per-pose blocks of many chunks (mixed path); the twiddles are restaged
@@ -2068,21 +2093,54 @@ int sxsk_fused_reduce(const sxsk_pose *poses, int npose, const float *part, int 
 	return cudaGetLastError();
 }
 
+/* Which form of the FP32 per-pose kernel: per pose, one row of P and 1 / (poses
+ * per combo) rows of R are read; all of R and the part of the tile's P rows
+ * beyond ~100 of the 129 MB of L2 come from DRAM.  Above 0.6 rows of those per
+ * pose the deep form is faster, below it the occupancy of the flat one is (it
+ * is bound by L2 there).  Flat / deep, ms:
+ *   L   Q    poses    DRAM rows   flat    deep
+ *   20  101   6,000   0.81        0.739   0.623
+ *   20  101  12,000   0.67        1.009   0.989
+ *   20  101  20,000   0.53        1.380   1.438
+ *   25  101  20,000   0.65        2.823   2.366
+ *   25  101  40,000   0.45        3.977   4.086
+ *   30  201  60,000   0.87       23.60   18.12
+ *   30  101 100,000   0.73       14.97   13.31
+ *   28  101 150,000   0.46       14.57   15.83
+ * A launch that fits the SMs at once only in the flat form keeps it (L = 15,
+ * Q = 51, 4,000 poses, 875 blocks: 0.143 and 0.160).  In a chain the deep form
+ * alone lets the next launch into its last wave, worth more than its 5 % at up
+ * to a few waves (eight dimers of 750 to 12,000 poses, L 10-25: phases of a
+ * batch 4.70 ms with it throughout, 5.23 by the rows' rule). */
+static bool pose_deep(int npose, int ncombo, int L, long blocks, bool chain)
+{
+	int K = L + 1, N = 2 * L + 1, NP = K * (K + 1) / 2, dev = 0, nsm = 0;
+	double tile = (double)K * N * NP * 3 * SXS_QT * sizeof(float2), miss = 1.0 - 100e6 / tile;
+	if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) return false;
+	if (chain && blocks <= 8L * POSE_FLAT * nsm) return true;
+	if ((double)ncombo / npose + (miss > 0.0 ? miss : 0.0) <= 0.6) return false;
+	return blocks <= (long)POSE_DEEP * nsm || blocks > (long)POSE_FLAT * nsm;
+}
+
 int sxsk_pose_cross(const sxsk_pose *poses, int npose, int combo_base, int ncombo, const void *P, const void *R,
-                    const double2 *tw, const void *cst, int Q, int L, void *cross, int fp32, cudaStream_t s)
+                    const double2 *tw, const void *cst, int Q, int L, void *cross, int fp32, int linked,
+                    cudaStream_t s)
 {
 	if (npose <= 0) return 0;
 	int NT = (Q + SXS_QT - 1) / SXS_QT;
 	long nb = (long)NT * ((npose + PC_PPB - 1) / PC_PPB);
 	if (nb > 0x7fffffffL) return cudaErrorInvalidValue;
-	if (fp32)
-		k_pose_cross<float, true><<<(unsigned)nb, 128, 0, s>>>(poses, npose, combo_base, ncombo, (const float2 *)P,
-		                                                  (const float2 *)R, tw, (const float2 *)cst, Q, L,
-		                                                  (float2 *)cross);
-	else
+	if (!fp32)
 		k_pose_cross<double, false><<<(unsigned)nb, 128, 0, s>>>(poses, npose, combo_base, ncombo, (const double2 *)P,
 		                                                   (const double2 *)R, tw, (const double *)cst, Q, L,
 		                                                   (double *)cross);
+	else if (pose_deep(npose, ncombo, L, nb, linked >= 0))
+		return chain_launch(k_pose_cross_deep, (unsigned)nb, 128, 0, s, linked > 0, poses, npose, combo_base, ncombo,
+		                    (const float2 *)P, (const float2 *)R, tw, (const float2 *)cst, Q, L, (float2 *)cross);
+	else
+		k_pose_cross<float, true><<<(unsigned)nb, 128, 0, s>>>(poses, npose, combo_base, ncombo, (const float2 *)P,
+		                                                  (const float2 *)R, tw, (const float2 *)cst, Q, L,
+		                                                  (float2 *)cross);
 	return cudaGetLastError();
 }
 

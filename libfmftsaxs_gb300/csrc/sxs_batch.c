@@ -628,7 +628,8 @@ static int launch_pieces(const blaunch *L, const char *hbase, int *nk, cudaStrea
 		} else if (L->kind == 2) {
 			const sxsk_pc_job *q = (const sxsk_pc_job *)hj + j;
 			rc = sxsk_pose_cross(q->poses, q->npose, q->combo_base, q->ncombo, q->P, q->R, q->tw, q->cst, q->Q, q->L,
-			                     q->cross, 1, s);
+			                     q->cross, 1, linked, s);
+			linked |= q->npose > 0;
 		} else {
 			const sxsk_fr_job *r = (const sxsk_fr_job *)hj + j;
 			rc = sxsk_fused_reduce(r->poses, r->npose, r->part, r->Q, r->L, r->cst, r->cross, s);

@@ -981,7 +981,7 @@ int sxs_plan_enqueue(sxsg_plan *p, int fit_mode, int timed)
 			if (timed) SXS_CU(cudaEventRecord(e[1], s));
 			SXS_K(sxsk_pose_cross(p->d_poses + p0, (int)(p1 - p0), (int)c0, (int)(c1 - c0), p->d_P, p->d_R, p->d_tw,
 			                      p->fp32 ? (const void *)p->d_cstf : (const void *)p->d_cst, Q, L,
-			                      p->d_cross, p->fp32, s));
+			                      p->d_cross, p->fp32, -1, s));
 		}
 		if (timed) SXS_CU(cudaEventRecord(e[2], s));
 		sxs_count_launches(sxsk_translate_launches(L) + 1);
