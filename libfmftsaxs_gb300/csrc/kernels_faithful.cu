@@ -505,10 +505,61 @@ __device__ __forceinline__ void tau_store(int2 *o, double v, double c28) { *o = 
  * = l + l1 (mod 2), in the same order, gives the same value bit for bit; the
  * signs of (-1)^m and i^p are exact and turn the sum into alternate sums and
  * differences of the products: two FP64 operations per term (four with the
- * signs multiplied in), 63 % of that pipe's rate at L = 30.  With the float
+ * signs multiplied in), 63 % of that pipe's rate at L = 30; one, where the
+ * sum is not stored as a double (tm_value).  With the float
  * form written here, not by a pass over a double table, 16 z of the mixed
  * path take 0.25 + 0.04 -> 0.20 ms at L = 20, Q = 101 and 2.14 + 0.29 -> 1.69
  * ms at L = 30, Q = 201. */
+/* sum over p = p0, p0 + 2, ..., p1 of +- dp[p] bp[p Q], the sign alternating
+ * from neg: products and sums rounded one by one */
+__device__ __forceinline__ double tm_sum(const double *dp, const double *bp, int Q, int p0, int p1, bool neg)
+{
+	double v = 0.0;
+	for (int p = p0; p <= p1; p += 2) {
+		double w = dp[p] * bp[(size_t)p * Q];
+		v = neg ? v - w : v + w;
+		neg = !neg;
+	}
+	return v;
+}
+
+/* What is stored as a float or as limbs is summed with fused multiply-adds
+ * (half the operations of the FP64 pipe, which bounds the kernel).  With
+ * n terms and partial sums of at most M the two sums differ by less than 4 n
+ * 2^-53 M, for a term is the difference of two partial sums; a float is
+ * therefore taken from the fused sum only if both ends of that interval
+ * round to it, and else from tm_sum: the stored floats are those of tm_sum.
+ * L = 30, Q = 201, 16 z: 1.69 -> 0.78 ms. */
+__device__ __forceinline__ double tm_fused(const double *dp, const double *bp, int Q, int p0, int p1, bool neg, int &top)
+{
+	double v = 0.0;
+	for (int p = p0; p <= p1; p += 2) {
+		double d = dp[p];
+		d = __hiloint2double(__double2hiint(d) ^ (neg ? 0x80000000 : 0), __double2loint(d));
+		v = __fma_rn(d, bp[(size_t)p * Q], v);
+		top = max(top, __double2hiint(v) & 0x7fffffff);
+		neg = !neg;
+	}
+	return v;
+}
+__device__ __forceinline__ double tm_value(double *, const double *dp, const double *bp, int Q, int p0, int p1, bool neg)
+{
+	return tm_sum(dp, bp, Q, p0, p1, neg);
+}
+__device__ __forceinline__ double tm_value(int2 *, const double *dp, const double *bp, int Q, int p0, int p1, bool neg)
+{
+	int top = 0;
+	return tm_fused(dp, bp, Q, p0, p1, neg, top);
+}
+__device__ __forceinline__ double tm_value(float *, const double *dp, const double *bp, int Q, int p0, int p1, bool neg)
+{
+	int top = 0;
+	double v = tm_fused(dp, bp, Q, p0, p1, neg, top);
+	/* M < the double whose high word is top + 1 */
+	double d = __hiloint2double(top + 1, 0) * ((2 * (p1 - p0) + 4) * 0x1p-53);
+	return (float)(v - d) == (float)(v + d) ? v : tm_sum(dp, bp, Q, p0, p1, neg);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128) k_tmatrix(const double *__restrict__ bes, const double *__restrict__ ds, int nz,
                                                  int Q, int L, const int2 *__restrict__ ll1, int nll1, int nbx,
@@ -531,11 +582,7 @@ __global__ void __launch_bounds__(128) k_tmatrix(const double *__restrict__ bes,
 		/* i^p: +1 (p % 4 == 0), -1 (2) for even p; the imaginary unit of i^p
 		 * for odd p: +1 (1), -1 (3); so the sign alternates with p */
 		bool neg = ((p0 & 2) != 0) != ((m & 1) != 0);
-		for (int p = p0; p <= l + l1; p += 2) {
-			double w = dp[p] * bp[(size_t)p * Q];
-			v = neg ? v - w : v + w;
-			neg = !neg;
-		}
+		v = tm_value(tau, dp, bp, Q, p0, l + l1, neg);
 	}
 	/* q-tiled: [tile][iz][m][l][l1][SXS_QT], tile = q / SXS_QT */
 	size_t base = (((size_t)(iq / SXS_QT) * nz + iz) * K + m) * K;
