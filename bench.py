@@ -188,7 +188,9 @@ class Clocks:
 # DRAM bytes per pose of the dominant kernel from ncu captures of the same
 # kernel on the poses of this workload with translation z index < 3 (the
 # same poses per translated row as the whole list, profiles/): the traffic
-# of a launch scales with the poses it processes at that density.
+# of a launch scales with the poses it processes at that density.  The FP64
+# figure is of the floating-point kernel; the fixed-point one reads rows of
+# the same size.
 TRAFFIC_PER_POSE = {("c1", "mixed"): 9.13e4, ("c1", "fp64"): 4.47e5}
 # L2-to-SM bytes per pose of the FP32 per-pose kernel (ncu
 # l1tex__m_xbar2l1tex_read_sectors on the same capture): the P row of every
@@ -197,8 +199,8 @@ L2_TO_SM_PER_POSE = {("c1", "mixed"): 6.18e5}
 
 
 def pose_flops(L, Q, precision):
-    """Algorithmic FLOPs of the per-pose contraction for one pose (both
-    precisions run the same kernel): over the (L+1)(L+2)/2 pairs
+    """Algorithmic FLOPs of the per-pose contraction for one pose (the same
+    count for both precisions): over the (L+1)(L+2)/2 pairs
     (m >= 0, l >= m) and Q q values, the phase w_m applied to the 3 channels
     of R (3 complex multiplies, 18 FLOPs) and the real parts of the 9
     channel products (36 FLOPs)."""
@@ -303,8 +305,10 @@ def accuracy(mix, ref, k=100, topk=None):
 
 def expansion_timing(g, w, fp64_peak):
     """The A_lm expansion per molecule (sxsg_expand, with its transfers of a
-    few MB) and its FP64 rate over the accumulation's 12 FLOPs per atom, q
-    and (l, m) (3 channels of complex-by-real multiply-adds)."""
+    few MB) and its rate over the accumulation's 12 FLOPs per atom, q and
+    (l, m) (3 channels of complex-by-real multiply-adds), as equivalent FP64
+    operations: the accumulation itself runs in fixed point on the integer
+    multiply-add pipe, so the fraction of the FP64 pipe's peak may pass 1."""
     out = {}
     water = g.ff_water()
     for name, m in (("receptor", w.rec), ("ligand", w.lig)):
@@ -665,7 +669,7 @@ def run_ours(args):
         "reference_flops_per_step": fref,
         "reference_equiv_tflops": fref / (ms * 1e-3) / 1e12,
         "roofline": {"bound": "fp32" if head == "mixed" else "fp64",
-                     "kernel": "k_pose_cross<%s>" % ("float" if head == "mixed" else "double"),
+                     "kernel": "k_pose_cross<float>" if head == "mixed" else "k_fix_cross",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak if peak > 0 else None,
                      "traffic": traffic,
@@ -673,8 +677,10 @@ def run_ours(args):
                                        "(z index < 1 for FP64), "
                                        "scaled to the poses of one launch (%d chunk(s) per run)" % nchunks,
                      "hbm_frac": (traffic * nchunks / (stage[2] * 1e-3) / 1e9 / 6773.5) if traffic else None,
-                     "peak_source": "measured in this run: register-resident %s FMA chains on every SM"
-                                    % ("FP32" if head == "mixed" else "FP64")},
+                     "peak_source": "measured in this run: register-resident FP32 FMA chains on every SM"
+                                    if head == "mixed" else
+                                    "measured in this run: register-resident FP64 FMA chains on every SM (the kernel "
+                                    "does the equivalent operations in fixed point on the integer pipe)"},
         "cpu_baseline": cpu_baseline_entry(w, cs, kind) if cs else None,
         "e2e": {"value": n / e2e_s, "unit": "poses/s", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": int(launches),
