@@ -23,6 +23,7 @@
  */
 #include "kernels.h"
 #include "chain.cuh"
+#include "smem.cuh"
 
 namespace {
 
@@ -206,11 +207,12 @@ __device__ __forceinline__ void rot_out(double2 y0, double2 A, double2 B, double
  * channel and accumulates its G gamma pairs in registers; with CH = 3 one
  * twiddle load and index step serve the three channels.  The padding
  * q >= Q is written as zeros. */
-/* the extended twiddles hs[N + (G-1) L] of a rotation block (all threads) */
+/* the extended twiddles hs[ROT_NTW] of a rotation block (all threads) */
+#define ROT_NTW(L, G) (2 * (L) + 1 + ((G) - 1) * (L))
 template <typename S, int G>
 __device__ __forceinline__ void rotate_stage(const double2 *__restrict__ tw, int L, RotTw<S> *hs)
 {
-	int N = 2 * L + 1, ne = N + (G - 1) * L;
+	int N = 2 * L + 1, ne = ROT_NTW(L, G);
 	for (int k = threadIdx.x; k < ne; k += blockDim.x) hs[k] = rot_tw<S>(tw, k, N);
 }
 
@@ -1750,21 +1752,16 @@ static int translate_slices(const void *U, const void *tau, const int32_t *combo
 	 * distinct banks */
 	int ts = K * SXS_QT, tgt = SXS_QT >= 16 ? 16 : 8;
 	while (ts % 32 != tgt) ts += SXS_QT;
-	size_t smem = (size_t)TR_PB * ts * (fp32 ? sizeof(float) : sizeof(double));
+	size_t elem = fp32 ? sizeof(float) : sizeof(double), smem = (size_t)TR_PB * ts * elem;
+	size_t most = (size_t)TR_PB * (SXS_LMAX_K * SXS_QT + 32) * elem;
 	if (fp32) {
-		if (smem > 48 * 1024) {
-			cudaError_t e = cudaFuncSetAttribute(k_translate<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                                     (int)smem);
-			if (e != cudaSuccess) return e;
-		}
+		cudaError_t e = smem_bound(k_translate<float>, smem, most);
+		if (e != cudaSuccess) return e;
 		k_translate<float><<<(unsigned)nb, 128, smem, s>>>((const float2 *)U, (const float *)tau, combo_zbg, slices,
 		                                                    nslice, cbase, ncombo, L, nzt, ts, (float2 *)R);
 	} else {
-		if (smem > 48 * 1024) {
-			cudaError_t e = cudaFuncSetAttribute(k_translate<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                                     (int)smem);
-			if (e != cudaSuccess) return e;
-		}
+		cudaError_t e = smem_bound(k_translate<double>, smem, most);
+		if (e != cudaSuccess) return e;
 		k_translate<double><<<(unsigned)nb, 128, smem, s>>>((const double2 *)U, (const double *)tau, combo_zbg,
 		                                                     slices, nslice, cbase, ncombo, L, nzt, ts,
 		                                                     (double2 *)R);
@@ -1777,18 +1774,16 @@ static int rotate_launch(const void *spf_t, const void *dtab, const double2 *tw,
                          cudaStream_t s)
 {
 	typedef typename Cx<S>::T V;
-	int K = L + 1, N = 2 * L + 1, NT = (Q + SXS_QT - 1) / SXS_QT;
+	int K = L + 1, NT = (Q + SXS_QT - 1) / SXS_QT;
 	/* three channels per thread in FP32 (one twiddle load for three) while
 	 * their 12 G accumulators leave room for warps (G <= 6, L <= 23: measured
 	 * 1.10 -> 1.04 ms at L = 20); FP64 is bound by its arithmetic pipe and
 	 * keeps one */
 	constexpr int CH = sizeof(S) == 4 ? 3 : 1;
-	size_t smem = sizeof(RotTw<S>) * (size_t)(N + (G - 1) * L);
+	size_t smem = sizeof(RotTw<S>) * (size_t)ROT_NTW(L, G);
 	auto kern = k_rotate<S, G, CH>;
-	if (smem > 48 * 1024) {
-		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		if (e != cudaSuccess) return e;
-	}
+	cudaError_t e = smem_bound(kern, smem, sizeof(RotTw<S>) * (size_t)ROT_NTW(SXS_LMAX_K - 1, G));
+	if (e != cudaSuccess) return e;
 	long nb = (long)K * K * NT;
 	if (nb > 0x7fffffffL) return cudaErrorInvalidValue;
 	kern<<<(unsigned)nb, ROT_THREADS(CH), smem, s>>>((const V *)spf_t, (const S *)dtab, tw, Q, L, conj, (V *)out);
@@ -1799,13 +1794,12 @@ template <int G>
 static int rotate2_launch(const void *spf_t, const void *dtab, const double2 *tw, int Q, int L, int conj, void *out,
                           cudaStream_t s)
 {
-	int K = L + 1, N = 2 * L + 1, NT = (Q + SXS_QT - 1) / SXS_QT;
-	size_t smem = ROT2_SMEM(L) + sizeof(RotTw<float>) * (size_t)(N + (G - 1) * L);
+	int K = L + 1, NT = (Q + SXS_QT - 1) / SXS_QT;
+	size_t smem = ROT2_SMEM(L) + sizeof(RotTw<float>) * (size_t)ROT_NTW(L, G);
 	auto kern = k_rotate2<G>;
-	if (smem > 48 * 1024) {
-		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		if (e != cudaSuccess) return e;
-	}
+	cudaError_t e = smem_bound(kern, smem, ROT2_SMEM(SXS_LMAX_K - 1) +
+	                                           sizeof(RotTw<float>) * (size_t)ROT_NTW(SXS_LMAX_K - 1, G));
+	if (e != cudaSuccess) return e;
 	long nb = (long)K * ((K + 1) / 2) * NT;
 	if (nb > 0x7fffffffL) return cudaErrorInvalidValue;
 	kern<<<(unsigned)nb, ROT2_THREADS, smem, s>>>((const float2 *)spf_t, (const float *)dtab, tw, Q, L, conj,
@@ -1879,8 +1873,8 @@ static int rotate_batch_launch(const sxsk_rot_job *jobs, const int4 *items, int 
 	size_t smem = sizeof(RotTw<float>) * (size_t)tw_max;
 	if (G >= ROT2_G) smem = (smem + 15) / 16 * 16 + ROT2_SMEM(l_max);
 	auto kern = k_rotate_batch<G>;
-	cudaError_t e = cudaSuccess;
-	if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	cudaError_t e = smem_bound(kern, smem, sizeof(RotTw<float>) * (size_t)ROT_NTW(SXS_LMAX_K - 1, G) + 16 +
+	                                           (G >= ROT2_G ? ROT2_SMEM(SXS_LMAX_K - 1) : 0));
 	int grid = 0;
 	if (!e) e = persistent_grid(kern, threads, smem, nitems, ctr, &grid);
 	if (e) return e;
@@ -2228,11 +2222,9 @@ int sxsk_fit_grid(const double *cross, const sxsk_pose *order, int slot0, int ns
 		if (smem <= 227 * 1024 || ppb == 1) break;
 		ppb = (ppb + 1) / 2;
 	}
-	if (smem > 227 * 1024) return cudaErrorInvalidValue;
-	if (smem > 48 * 1024) {
-		cudaError_t e = cudaFuncSetAttribute(k_fit_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		if (e != cudaSuccess) return e;
-	}
+	if (smem > SXS_SMEM_MAX) return cudaErrorInvalidValue;
+	cudaError_t e = smem_bound(k_fit_grid, smem, SXS_SMEM_MAX);
+	if (e != cudaSuccess) return e;
 	long ngroup = (nslot + ppb - 1) / ppb;
 	int grid_n = (int)(ngroup < (long)max_blocks || max_blocks <= 0 ? ngroup : max_blocks);
 	k_fit_grid<<<grid_n, FIT_THREADS, smem, s>>>(cross, order, slot0, nslot, Q, fc, a0sum, peak, gtab, c1g, n1, c2g,

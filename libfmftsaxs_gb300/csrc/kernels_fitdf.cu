@@ -18,6 +18,7 @@
  * fitdf_core.h must not be contracted.
  */
 #include "kernels.h"
+#include "smem.cuh"
 #include "fitdf_core.h"
 
 #include <string.h>
@@ -303,10 +304,8 @@ extern "C" int sxsk_fit_grid_df(const float2 *cross, const sxsk_pose *order, int
 	J.cross = cross; J.order = order; J.fc = fc; J.gdf = gdf; J.c1g = c1g; J.c2g = c2g;
 	J.chi = chi; J.c1 = c1; J.c2 = c2; J.cell = cell; J.grid = grid;
 	J.a0sum = a0sum; J.peak = peak; J.slot0 = slot0; J.nslot = nslot; J.Q = Q; J.n1 = n1; J.n2 = n2;
-	if (smem > 48 * 1024) {
-		cudaError_t e = cudaFuncSetAttribute(k_fit_grid_df, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		if (e != cudaSuccess) return e;
-	}
+	cudaError_t e = smem_bound(k_fit_grid_df, smem, SXS_SMEM_MAX);
+	if (e != cudaSuccess) return e;
 	long ngroup = (nslot + J.ppb - 1) / J.ppb;
 	int grid_n = (int)(ngroup < (long)max_blocks || max_blocks <= 0 ? ngroup : max_blocks);
 	k_fit_grid_df<<<grid_n, FITD_THREADS, smem, s>>>(J);
@@ -317,9 +316,7 @@ extern "C" int sxsk_fit_grid_df_batch(const sxsk_fit_job *jobs, const int2 *item
                                       cudaStream_t s)
 {
 	if (nitems <= 0) return 0;
-	cudaError_t e = cudaSuccess;
-	if (smem > 48 * 1024)
-		e = cudaFuncSetAttribute(k_fit_grid_df_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	cudaError_t e = smem_bound(k_fit_grid_df_batch, smem, SXS_SMEM_MAX - 16);
 	int dev = 0, nsm = 0, per = 1;
 	if (!e) e = cudaGetDevice(&dev);
 	if (!e) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

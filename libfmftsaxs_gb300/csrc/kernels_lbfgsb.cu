@@ -18,6 +18,7 @@
  * latency.  Now 4.1 and 2.0 ms, the evaluations ~2.4 ms of FP64 pipe.)
  */
 #include "kernels.h"
+#include "smem.cuh"
 #include "lbfgsb_core.h"
 
 #include <type_traits>
@@ -232,6 +233,7 @@ __global__ void k_lbfgsb_thread(const double *__restrict__ cross, int npose, int
 }
 
 #define LB_MAX_EVAL 100000
+#define LB_SMEM_MAX (225 * 1024)   /* dynamic; the slots' points and sums have 1.1 KB beside it */
 
 template <typename T, int LBT>
 int lbfgsb_launch(const T *cross, int npose, int Q, const double *q, const double *a, double mult, double peak,
@@ -240,7 +242,7 @@ int lbfgsb_launch(const T *cross, int npose, int Q, const double *q, const doubl
 {
 	int per = 0;
 	auto kern = k_lbfgsb<T, LBT>;
-	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	cudaError_t e = smem_bound(kern, smem, LB_SMEM_MAX);
 	if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, LBT, smem);
 	if (e) return (int)e;
 	if (per < 1) return (int)cudaErrorInvalidConfiguration;
@@ -276,7 +278,7 @@ int lbfgsb_any(const T *cross, int npose, int Q, const double *q, const double *
 		smem = sizeof(double) * (9 * (size_t)Q + (size_t)slots * LB_ROWS * (Q | 1));
 		if (smem <= 110 * 1024 || slots == 1) break;
 	}
-	if (smem > 225 * 1024) {
+	if (smem > LB_SMEM_MAX) {
 		if (rescale || !std::is_same<T, double>::value)
 			return (int)cudaErrorInvalidValue;   /* plans have at most 1,024 q */
 		k_lbfgsb_thread<<<(npose + 63) / 64, 64, 0, s>>>((const double *)cross, npose, Q, q, a, mult, LB_MAX_EVAL, chi, c1,

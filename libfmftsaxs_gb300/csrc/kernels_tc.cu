@@ -28,6 +28,7 @@
  * status 2 the CUDA context itself must be considered unusable.
  */
 #include "kernels.h"
+#include "smem.cuh"
 
 #include <stdint.h>
 
@@ -307,7 +308,7 @@ extern "C" int sxsk_rotate_tc(const void *spf_t, const float *dtabf, const doubl
 	if (smem > 227 * 1024) return cudaErrorInvalidValue;
 	int ae = TC_M * KP;
 	k_tc_amat<<<(ae + 255) / 256, 256, 0, s>>>(tw, L, KP, amat, amat + ae);
-	cudaError_t e = cudaFuncSetAttribute(k_rotate_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	cudaError_t e = smem_bound(k_rotate_tc, smem, SXS_SMEM_MAX);
 	if (e != cudaSuccess) return e;
 	int dev = 0, nsm = 0;
 	cudaGetDevice(&dev);

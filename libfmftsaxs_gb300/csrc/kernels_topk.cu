@@ -20,6 +20,7 @@
  * its launches without a host round trip.
  */
 #include "kernels.h"
+#include "smem.cuh"
 
 #include <stdint.h>
 
@@ -257,10 +258,8 @@ int sxsk_topk(const double *chi, const double *c1, const double *c2, long n, int
 	int kp = 1;
 	while (kp < k) kp <<= 1;
 	size_t smem = (size_t)kp * (sizeof(unsigned long long) + sizeof(unsigned int));
-	if (smem > 48 * 1024) {
-		cudaError_t e = cudaFuncSetAttribute(k_topk_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		if (e) return e;
-	}
+	cudaError_t e = smem_bound(k_topk_sort, smem, SXS_SMEM_MAX);
+	if (e) return e;
 	k_topk_sort<<<1, 1024, smem, s>>>(okey, opos, k, kp, chi, c1, c2, out_pos, out_chi, out_c1, out_c2);
 	return cudaGetLastError();
 }
