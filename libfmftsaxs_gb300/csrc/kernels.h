@@ -102,8 +102,8 @@ size_t sxsk_rotate_tc_scratch(int L);
 
 /* The plain path's contractions in fixed point (kernels_fixed.cu), L <=
  * SXSK_FIX_LMAX: tables of the FP64 layouts and sizes whose complex entries
- * are limbs {re h, re l, im h, im l} (int4), scaled per molecule and q.
- * molecule: sc[2][Qp] (Qp = Q rounded up to 8) = {2^(28 - e), 2^e} of the
+ * are limbs {re h, re l, im h, im l} (int4), scaled per molecule, channel
+ * and q.  molecule: sc[3][Qp] (Qp = Q rounded up to 8) = 2^(28 - e) of the
  * flat coefficients, spf [3][K2][Q] their limbs (conjugated when conj);
  * two launches.  dtab: limbs of a Wigner-d table.  nu: nu2[nz][Qp] = powers of
  * two that bound the translation matrices' norms. */

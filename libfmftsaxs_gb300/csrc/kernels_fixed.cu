@@ -7,22 +7,25 @@
  * T/s over the GPU); its 32 x 32 + 64-bit integer multiply-add (IMAD.WIDE)
  * takes 28 (4.6 clocks per warp and scheduler).  A real number v of a table
  * row is held as v / 2^e = (h 2^29 + l) 2^-57 with two 32-bit limbs, |l| <=
- * 2^28, and one exponent e per molecule and q for the whole row; a product
- * is then three IMAD.WIDE,
+ * 2^28, and one exponent e per molecule, channel and q; a product is then
+ * three IMAD.WIDE,
  *   h h' -> a 64-bit sum, h l' + l h' -> a second 64-bit sum
  * (l l', at most 2^-58 of the first sum's scale, is dropped), and the sums are
  * exact: nothing is rounded until a sum is complete.
  *
  * The exponents come from norms that the operations keep: a rotation leaves
- * the 2-norm of a molecule's coefficients at each q alone, so bounds of
- * |A(q)|_2 hold for every row of the rotated tables, and the translation by z
- * is a compression of the multiplication by f(t) = exp(i q z t), so that its
+ * the 2-norm of a channel's coefficients at each q alone, so bounds of
+ * |A_c(q)|_2 hold for every row of the rotated tables, and the translation by
+ * z is a compression of the multiplication by f(t) = exp(i q z t), so that its
  * norm is at most max |f|, taken from the Bessel values in use.  With
  * Cauchy-Schwarz no sum overflows, and an entry is off by 2^-58 of its row's
  * bound, where FP64 rounds every term and partial sum at 2^-53 of its size:
- * against long double the cross terms are no further off than those of the
- * FP64 kernels (tests/test_gpu_fixed.py).  A norm that is not finite makes
- * the scale, and with it the result, NaN.
+ * against long double, and relative to the norms of its own two channels, no
+ * channel pair's cross term is further off than the FP64 kernels' (rms over
+ * poses; tests/test_gpu_fixed_channels.py has channels weaker than the others
+ * by up to 1e6).  The exponents are a molecule's own: its rotation table
+ * serves any partner.  A norm that is not finite makes all six terms of its q
+ * NaN.
  */
 #include "kernels.h"
 #include "chain.cuh"
@@ -68,21 +71,22 @@ __device__ __forceinline__ int4 entry(i64 x, i64 y)
 	return make_int4(xh, lo_limb(x, xh), yh, lo_limb(y, yh));
 }
 
-/* sc[0][q] = 2^(28 - e), sc[1][q] = 2^e of a molecule's coefficients (host
- * flat layout [3][Q][K2][2]), NaN where a norm is not finite.  The norms of
- * two channels add up to at most 2^(e + 1) / 1.15: the per-pose kernel adds two
- * channels' entries in 32 bits, and the translation may lengthen a row by
- * up to 1.12.  A block per q, padded with ones up to Qp. */
+/* sc[ch][q] = 2^(28 - e) of a molecule's coefficients (host flat layout
+ * [3][Q][K2][2]), with the channel's norm at most 2^(e + 1) / 1.15, which
+ * leaves room for the translation to lengthen a row by up to 1.12; NaN at all
+ * three where a norm is not finite.  A channel without entries has the
+ * smallest e.  A block per q, padded with ones up to Qp. */
+#define FIX_EMAX 900
 __global__ void __launch_bounds__(128) k_fix_scale(const double *__restrict__ flat, int Q, int K2, int Qp,
                                                    double *__restrict__ sc)
 {
 	__shared__ double part[4];
 	int q = blockIdx.x;
 	if (q >= Q) {
-		if (threadIdx.x == 0) sc[q] = sc[Qp + q] = 1.0;
+		if (threadIdx.x < 3) sc[threadIdx.x * Qp + q] = 1.0;
 		return;
 	}
-	double big = 0.0, next = 0.0;
+	double c28[3];
 	bool bad = false;
 	for (int ch = 0; ch < 3; ch++) {
 		const double *a = flat + ((size_t)ch * Q + q) * K2 * 2;
@@ -91,30 +95,23 @@ __global__ void __launch_bounds__(128) k_fix_scale(const double *__restrict__ fl
 		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
 		if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = s;
 		__syncthreads();
-		s = sqrt(part[0] + part[1] + part[2] + part[3]);
+		s = 0.575 * sqrt(part[0] + part[1] + part[2] + part[3]);
 		__syncthreads();
-		bad |= !isfinite(s);
-		if (s > big) {
-			next = big;
-			big = s;
-		} else {
-			next = fmax(next, s);
-		}
+		int e = -FIX_EMAX;
+		if (!isfinite(s)) bad = true;
+		else if (s > 0.0) frexp(s, &e);               /* s < 2^e */
+		c28[ch] = ldexp(1.0, 28 - min(max(e, -FIX_EMAX), FIX_EMAX));
 	}
-	if (threadIdx.x == 0) {
-		int e = 0;
-		double t = 0.575 * (big + next);
-		if (t > 0.0 && !bad) frexp(t, &e);            /* t < 2^e */
-		e = e < -900 ? -900 : (e > 900 ? 900 : e);
-		sc[q] = bad ? nan("") : ldexp(1.0, 28 - e);
-		sc[Qp + q] = bad ? nan("") : ldexp(1.0, e);
-	}
+	if (threadIdx.x == 0)
+		for (int ch = 0; ch < 3; ch++) sc[ch * Qp + q] = bad ? nan("") : c28[ch];
 }
+/* e of a scale 2^(28 - e) */
+__device__ __forceinline__ int fix_exp(double c28) { return 28 + 1023 - (__double2hiint(c28) >> 20); }
 
 /* [3][Q][K2][2] -> [3][K2][Q] limbs {re h, re l, im h, im l}, conjugated
  * when conj != 0 */
-__global__ void k_fix_spf(const double *__restrict__ flat, const double *__restrict__ sc, int Q, int K2, int conj,
-                          int4 *__restrict__ t)
+__global__ void k_fix_spf(const double *__restrict__ flat, const double *__restrict__ sc, int Q, int K2, int Qp,
+                          int conj, int4 *__restrict__ t)
 {
 	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= 3L * Q * K2) return;
@@ -122,7 +119,8 @@ __global__ void k_fix_spf(const double *__restrict__ flat, const double *__restr
 	long r = i / Q;
 	int lm = (int)(r % K2), ch = (int)(r / K2);
 	const double *s = flat + (((size_t)ch * Q + iq) * K2 + lm) * 2;
-	int2 a = sxs_limbs(s[0], sc[iq]), b = sxs_limbs(conj ? -s[1] : s[1], sc[iq]);
+	double c28 = sc[ch * Qp + iq];
+	int2 a = sxs_limbs(s[0], c28), b = sxs_limbs(conj ? -s[1] : s[1], c28);
 	t[i] = make_int4(a.x, a.y, b.x, b.y);
 }
 
@@ -388,6 +386,9 @@ k_fix_translate(const int4 *__restrict__ U, const int2 *__restrict__ tau, const 
 	chain_end();
 }
 
+/* 2^e for a normal result */
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
 /* 16-byte loads with L2 policies: receptor rows are read by many poses
  * (evict_last), translated rows by the few poses of their combo
  * (evict_first) */
@@ -407,16 +408,11 @@ __device__ __forceinline__ int4 ld_pol(const int4 *p, uint64_t pol)
 	return v;
 }
 
-__device__ __forceinline__ int4 operator+(int4 a, int4 b)
-{
-	return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-}
-
-/* (re, im) += p r for complex limbs */
-__device__ __forceinline__ void cmul_add(Acc &re, Acc &im, int4 p, int4 r)
+/* (re, im) += p r for complex limbs, n = -Im p */
+__device__ __forceinline__ void cmul_add(Acc &re, Acc &im, int4 p, int2 n, int4 r)
 {
 	mul_add(re, p.x, p.y, r.x, r.y);
-	mul_add(re, p.z, p.w, -r.z, -r.w);
+	mul_add(re, n.x, n.y, r.z, r.w);
 	mul_add(im, p.x, p.y, r.z, r.w);
 	mul_add(im, p.z, p.w, r.x, r.y);
 }
@@ -424,18 +420,27 @@ __device__ __forceinline__ void cmul_add(Acc &re, Acc &im, int4 p, int4 r)
 #define FPC_POSES 16
 #define FPC_THREADS (FPC_POSES * SXS_QT)
 
+/* x + y 2^-d for d >= 0 and x 2^d + y below, rounded: two sums of a channel
+ * pair in the unit of the larger one */
+__device__ __forceinline__ i64 join(i64 x, i64 y, int d)
+{
+	i64 big = d < 0 ? y : x, small = d < 0 ? x : y;
+	int k = min(abs(d), 62);
+	return big + ((small + ((1ll << k) >> 1)) >> k);
+}
+
 /* Per-pose cross terms from limbs.  Thread = (pose, q); block = 16
  * consecutive poses (sorted by combo) x the 8 q of a tile, tile-major.
- * Per m the six channel sums over l are complex,
- *   P_a R_b + P_b R_a = (P_a + P_b)(R_a + R_b) - P_a R_a - P_b R_b,
- * so six complex products (72 IMAD.WIDE and 36 adds) replace nine; the
- * pose's phase w_m is applied once per m, to the sums, and the subtraction
- * once per pose.  Bound by IMAD.WIDE: 333 of the 420 clocks per pair and warp.
- * At L = 20, Q = 101, 70,000 poses: 19.0 ms (FP64 kernel: 87.5).  Measured
- * beside it: nine products 26.5; three real products per complex one
- * (Karatsuba; 168 registers) 20.3; no prefetch of the next pair 21.4; the mixed
- * products h l' + l h' as FP32 sums 15.3, but then the result is up to 1.3
- * times (L = 1: twice) as far off as the FP64 kernels'. */
+ * Per m the nine channel products are summed over l as complex numbers, the
+ * two of a pair (P_a R_b and P_b R_a, whose units differ) joined in the larger
+ * unit, and the pose's phase w_m is applied to the six sums.  Bound by
+ * the integer pipe: 108 IMAD.WIDE per pair of rows.  At L = 20, Q = 101,
+ * 70,000 poses: 25.1 ms (FP64 kernel: 87.5).  With one unit for all channels
+ * six products do, (P_a + P_b)(R_a + R_b) - P_a R_a - P_b R_b, in 18.9 ms, but
+ * a channel ten times weaker then has up to 7 times the FP64 kernels' error
+ * (a thousand times: 500); the same six with one operand of each sum shifted to
+ * the other's unit 26.1; a thread per channel of P 26.9; Im P negated once
+ * instead of Im R 25.1 against 25.7; two blocks per SM 28.7. */
 __global__ void __launch_bounds__(FPC_THREADS, 3)
 k_fix_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int ncombo,
             const int32_t *__restrict__ combo_zbg, const int4 *__restrict__ P, const int4 *__restrict__ R,
@@ -459,14 +464,27 @@ k_fix_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int 
 	const int4 *Pr = P + (((size_t)t * nrow + ps.b1 * N + ps.g1) * NP) * 3 * SXS_QT + qq;
 	const int4 *Rr = R + (((size_t)t * ncombo + ps.combo - combo_base) * NP) * 3 * SXS_QT + qq;
 	uint64_t polP = fix_policy(true), polR = fix_policy(false);
+	const int ca[6] = {0, 0, 0, 1, 1, 2}, cb[6] = {0, 1, 2, 1, 2, 2};
+	double nu = nu2[(size_t)combo_zbg[3 * (ps.combo - combo_base)] * Qp + q], ok = nu;
+	int eA[3], eB[3], d[3];
+#pragma unroll
+	for (int c = 0; c < 3; c++) {
+		double a = scA[c * Qp + q], b = scB[c * Qp + q];
+		eA[c] = fix_exp(a);
+		eB[c] = fix_exp(b);
+		ok += a + b;
+	}
+	d[0] = eA[0] + eB[1] - eA[1] - eB[0];
+	d[1] = eA[0] + eB[2] - eA[2] - eB[0];
+	d[2] = eA[1] + eB[2] - eA[2] - eB[1];
 	int e = 0;
 	int4 p0 = ld_pol(Pr, polP), p1 = ld_pol(Pr + SXS_QT, polP), p2 = ld_pol(Pr + 2 * SXS_QT, polP);
 	int4 r0 = ld_pol(Rr, polR), r1 = ld_pol(Rr + SXS_QT, polR), r2 = ld_pol(Rr + 2 * SXS_QT, polR);
 	int left = NP;
 	for (int m = 0; m < K; m++) {
-		Acc re[6], im[6];
+		Acc re[9], im[9];
 #pragma unroll
-		for (int c = 0; c < 6; c++) re[c] = im[c] = acc0();
+		for (int c = 0; c < 9; c++) re[c] = im[c] = acc0();
 		for (int i = K - m; i > 0; i--) {
 			int4 a0 = p0, a1 = p1, a2 = p2, b0 = r0, b1 = r1, b2 = r2;
 			/* the next pair's rows stream in behind this pair's products */
@@ -479,19 +497,29 @@ k_fix_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int 
 			r0 = ld_pol(Rr, polR);
 			r1 = ld_pol(Rr + SXS_QT, polR);
 			r2 = ld_pol(Rr + 2 * SXS_QT, polR);
-			cmul_add(re[0], im[0], a0, b0);
-			cmul_add(re[3], im[3], a1, b1);
-			cmul_add(re[5], im[5], a2, b2);
-			cmul_add(re[1], im[1], a0 + a1, b0 + b1);
-			cmul_add(re[2], im[2], a0 + a2, b0 + b2);
-			cmul_add(re[4], im[4], a1 + a2, b1 + b2);
+			int2 n0 = make_int2(-a0.z, -a0.w), n1 = make_int2(-a1.z, -a1.w), n2 = make_int2(-a2.z, -a2.w);
+			cmul_add(re[0], im[0], a0, n0, b0);
+			cmul_add(re[1], im[1], a0, n0, b1);
+			cmul_add(re[2], im[2], a0, n0, b2);
+			cmul_add(re[3], im[3], a1, n1, b1);
+			cmul_add(re[4], im[4], a1, n1, b2);
+			cmul_add(re[5], im[5], a2, n2, b2);
+			cmul_add(re[6], im[6], a1, n1, b0);
+			cmul_add(re[7], im[7], a2, n2, b0);
+			cmul_add(re[8], im[8], a2, n2, b1);
 		}
 		/* F += Re(w_m G): the sums start with m = 0, which counts once where
 		 * the others count twice (their mirror images) */
 		int4 w = tws[e];
 #pragma unroll
 		for (int c = 0; c < 6; c++) {
+			const int o[6] = {0, 6, 7, 0, 8, 0};              /* the pair's other product */
 			i64 x = value(re[c]), y = value(im[c]);
+			if (o[c]) {
+				int dd = d[c == 4 ? 2 : c - 1];
+				x = join(x, value(re[o[c]]), dd);
+				y = join(y, value(im[o[c]]), dd);
+			}
 			int xh = hi_limb(x), xl = lo_limb(x, xh), yh = hi_limb(y), yl = lo_limb(y, yh);
 			Acc f = {0, 0};
 			if (m > 0) f = {F[c][threadIdx.x], F[6 + c][threadIdx.x]};
@@ -508,17 +536,16 @@ k_fix_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int 
 		e += ps.a2;
 		if (e >= N) e -= N;
 	}
-	double s = scA[Qp + q] * scB[Qp + q] * nu2[(size_t)combo_zbg[3 * (ps.combo - combo_base)] * Qp + q] * 0x1p-55;
 	double *o = cross + (size_t)ps.src * 6 * Q + q;
-	const int ca[6] = {0, 0, 0, 3, 3, 5}, cb[6] = {0, 3, 5, 3, 5, 5};
 #pragma unroll
 	for (int c = 0; c < 6; c++) {
 		i64 hh = F[c][threadIdx.x], mid = F[6 + c][threadIdx.x];
-		if (ca[c] != cb[c]) {
-			hh -= F[ca[c]][threadIdx.x] + F[cb[c]][threadIdx.x];
-			mid -= F[6 + ca[c]][threadIdx.x] + F[6 + cb[c]][threadIdx.x];
-		}
-		o[(size_t)c * Q] = fma(s, (double)(2 * hh + ((mid + (1 << 27)) >> 28)), cst[(size_t)c * Q + q]);
+		/* the pair's unit, in two factors that cannot overflow */
+		int ex = max(eA[ca[c]] + eB[cb[c]], eA[cb[c]] + eB[ca[c]]) + (__double2hiint(nu) >> 20) - 1023 - 55;
+		int ea = ex / 2, eb = ex - ea;
+		double v = (double)(2 * hh + ((mid + (1 << 27)) >> 28)) * pow2(ea);
+		if (isnan(ok)) v = ok;
+		o[(size_t)c * Q] = fma(v, pow2(eb), cst[(size_t)c * Q + q]);
 	}
 }
 
@@ -568,7 +595,7 @@ int sxsk_fix_molecule(const double *flat, int Q, int L, int conj, double *sc, vo
 {
 	int K2 = (L + 1) * (L + 1), Qp = (Q + SXS_QT - 1) / SXS_QT * SXS_QT;
 	k_fix_scale<<<Qp, 128, 0, s>>>(flat, Q, K2, Qp, sc);
-	k_fix_spf<<<nblk(3L * Q * K2, 256), 256, 0, s>>>(flat, sc, Q, K2, conj, (int4 *)spf);
+	k_fix_spf<<<nblk(3L * Q * K2, 256), 256, 0, s>>>(flat, sc, Q, K2, Qp, conj, (int4 *)spf);
 	return cudaGetLastError();
 }
 

@@ -836,9 +836,9 @@ void sxs_plan_mark_run(sxsg_plan *p, int fit_mode, const float *ms)
 }
 
 /* The contraction tables of a run.  On the plain path the fixed-point kernels
- * (kernels_fixed.cu) take a quarter of the FP64 ones' time (L = 20, Q = 101,
- * 70,000 poses: tables 4.0 against 17.0 ms, translation 16.0 / 59.2, poses
- * 19.0 / 87.5) and are as close to the exact sums; they hold a column in
+ * (kernels_fixed.cu) take less than a third of the FP64 ones' time (L = 20, Q
+ * = 101, 70,000 poses: tables 4.0 against 17.0 ms, translation 16.0 / 59.2,
+ * poses 25.1 / 87.5) and are as close to the exact sums; they hold a column in
  * registers up to L = 31.  The L-BFGS-B fit keeps the FP64 kernels: its stopping point
  * moves by up to 1e-6 in (c1, c2) when the last bits of its input change. */
 int sxs_plan_table_form(int L, int precision, int fit_mode)
@@ -855,8 +855,8 @@ static int plan_fixed_inputs(sxsg_plan *p)
 	cudaStream_t s = p->s;
 	if (!p->d_nu2 && p->nzt > 0) SXS_CU(cudaMallocAsync((void **)&p->d_nu2, sizeof(double) * Qp * p->nzt, s));
 	if (p->d_Bx) return 0;
-	if (!p->d_scA) SXS_CU(cudaMallocAsync((void **)&p->d_scA, sizeof(double) * 2 * Qp, s));
-	if (!p->d_scB) SXS_CU(cudaMallocAsync((void **)&p->d_scB, sizeof(double) * 2 * Qp, s));
+	if (!p->d_scA) SXS_CU(cudaMallocAsync((void **)&p->d_scA, sizeof(double) * 3 * Qp, s));
+	if (!p->d_scB) SXS_CU(cudaMallocAsync((void **)&p->d_scB, sizeof(double) * 3 * Qp, s));
 	if (!p->d_Ax) SXS_CU(cudaMallocAsync(&p->d_Ax, sizeof(int4) * n, s));
 	SXS_K(sxsk_fix_molecule(p->d_A, p->Q, p->L, 0, p->d_scA, p->d_Ax, s));
 	SXS_CU(cudaMallocAsync(&p->d_Bx, sizeof(int4) * n, s));
