@@ -24,8 +24,8 @@
  * channel pair's cross term is further off than the FP64 kernels' (rms over
  * poses; tests/test_gpu_fixed_channels.py has channels weaker than the others
  * by up to 1e6).  The exponents are a molecule's own: its rotation table
- * serves any partner.  A norm that is not finite makes all six terms of its q
- * NaN.
+ * serves any partner.  A coefficient that is not finite makes all six terms
+ * of its q NaN.
  */
 #include "kernels.h"
 #include "chain.cuh"
@@ -71,36 +71,55 @@ __device__ __forceinline__ int4 entry(i64 x, i64 y)
 	return make_int4(xh, lo_limb(x, xh), yh, lo_limb(y, yh));
 }
 
+/* 2^e for a normal result */
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
 /* sc[ch][q] = 2^(28 - e) of a molecule's coefficients (host flat layout
  * [3][Q][K2][2]), with the channel's norm at most 2^(e + 1) / 1.15, which
  * leaves room for the translation to lengthen a row by up to 1.12; NaN at all
- * three where a norm is not finite.  A channel without entries has the
- * smallest e.  A block per q, padded with ones up to Qp. */
-#define FIX_EMAX 900
+ * three where a coefficient is not finite.  The norm is formed of the
+ * coefficients over their largest exponent: squares neither overflow nor
+ * vanish.  e is at least FIX_EMIN (the scale is a double); a channel without
+ * entries has that.  A block per q, padded with ones up to Qp. */
+#define FIX_EMIN (-995)
 __global__ void __launch_bounds__(128) k_fix_scale(const double *__restrict__ flat, int Q, int K2, int Qp,
                                                    double *__restrict__ sc)
 {
 	__shared__ double part[4];
+	__shared__ int top[3];
 	int q = blockIdx.x;
 	if (q >= Q) {
 		if (threadIdx.x < 3) sc[threadIdx.x * Qp + q] = 1.0;
 		return;
 	}
+	if (threadIdx.x < 3) top[threadIdx.x] = 0;
+	__syncthreads();
 	double c28[3];
 	bool bad = false;
 	for (int ch = 0; ch < 3; ch++) {
 		const double *a = flat + ((size_t)ch * Q + q) * K2 * 2;
-		double s = 0.0;
-		for (int i = threadIdx.x; i < 2 * K2; i += blockDim.x) s = fma(a[i], a[i], s);
+		int h = 0;                                    /* largest high word: exponent and leading bits */
+		for (int i = threadIdx.x; i < 2 * K2; i += blockDim.x) h = max(h, __double2hiint(a[i]) & 0x7fffffff);
+		h = __reduce_max_sync(0xffffffffu, h);
+		if (threadIdx.x % 32 == 0) atomicMax(&top[ch], h);
+		__syncthreads();
+		int k = (top[ch] >> 20) - 1022, e = FIX_EMIN;  /* |a| < 2^k */
+		bad |= k > 1024;
+		double f = pow2(-k / 2), g = pow2(-k - -k / 2), s = 0.0;
+		for (int i = threadIdx.x; i < 2 * K2; i += blockDim.x) {
+			double v = a[i] * f * g;
+			s = fma(v, v, s);
+		}
 		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
 		if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = s;
 		__syncthreads();
 		s = 0.575 * sqrt(part[0] + part[1] + part[2] + part[3]);
 		__syncthreads();
-		int e = -FIX_EMAX;
-		if (!isfinite(s)) bad = true;
-		else if (s > 0.0) frexp(s, &e);               /* s < 2^e */
-		c28[ch] = ldexp(1.0, 28 - min(max(e, -FIX_EMAX), FIX_EMAX));
+		if (s > 0.0) {
+			frexp(s, &e);                             /* s < 2^e */
+			e = max(e + k, FIX_EMIN);
+		}
+		c28[ch] = pow2(28 - e);
 	}
 	if (threadIdx.x == 0)
 		for (int ch = 0; ch < 3; ch++) sc[ch * Qp + q] = bad ? nan("") : c28[ch];
@@ -385,9 +404,6 @@ k_fix_translate(const int4 *__restrict__ U, const int2 *__restrict__ tau, const 
 	}
 	chain_end();
 }
-
-/* 2^e for a normal result */
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
 /* 16-byte loads with L2 policies: receptor rows are read by many poses
  * (evict_last), translated rows by the few poses of their combo
