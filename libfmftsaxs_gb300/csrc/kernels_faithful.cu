@@ -410,15 +410,16 @@ __global__ void __launch_bounds__(EXP_THREADS, 10) k_expand_fix(const int4 *__re
 			if (t % 32 == 0) atomicMax(&emax[c], v);
 		}
 		__syncthreads();
-		for (int c = 0; c < 3; c++) em[c] = emax[c];
-		/* w = M 2^(E - 1075) -> M >> (emax - E), rounded: unit 2^(emax - 1075) */
+		for (int c = 0; c < 3; c++) em[c] = max(emax[c], 1);
+		/* w = M 2^(E - 1075) -> M >> (emax - E), rounded: unit 2^(emax - 1075);
+		 * subnormal numbers have the exponent 1 without the leading bit */
 		for (int k = t; k < na; k += EXP_THREADS)
 #pragma unroll
 			for (int c = 0; c < 3; c++) {
 				long long b = w[c][k];
-				int E = (int)(b >> 52) & 0x7ff, s = em[c] - E;
-				long long M = (b & 0xfffffffffffffll) | 0x10000000000000ll;
-				M = E == 0 || s > 53 ? 0 : (s > 0 ? (M + (1ll << (s - 1))) >> s : M);
+				int E = (int)(b >> 52) & 0x7ff, s = em[c] - max(E, 1);
+				long long M = (b & 0xfffffffffffffll) | (E ? 0x10000000000000ll : 0);
+				M = s > 53 ? 0 : (s > 0 ? (M + (1ll << (s - 1))) >> s : M);
 				if (b < 0) M = -M;
 				int h = (int)((M + (1ll << 26)) >> 27), lo = (int)((unsigned)M - ((unsigned)h << 27));
 				w[c][k] = (long long)(((unsigned long long)(unsigned)lo << 32) | (unsigned)h);
@@ -445,8 +446,9 @@ __global__ void __launch_bounds__(EXP_THREADS, 10) k_expand_fix(const int4 *__re
 			for (int c = 0; c < 6; c++) {
 				/* hh 2^54 + mid 2^27 in units of 2^(emax - 1075) 2^(y_exp - 54) */
 				int e = em[c / 2], s2 = e - 1075 + y_exp(l);
-				double u = e == 0x7ff ? nan("") : (s2 > -1022 ? exp2i(s2) : 0.0);
-				a6[c] = fma(to_double(hh[c] + ((mid[c] + (1 << 26)) >> 27)), u, a6[c]);
+				double v = to_double(hh[c] + ((mid[c] + (1 << 26)) >> 27));
+				if (s2 > -1022) a6[c] = fma(v, e == 0x7ff ? nan("") : exp2i(s2), a6[c]);
+				else a6[c] = a6[c] + v * exp2i(s2 + 512) * 0x1p-512;
 			}
 		}
 		__syncthreads();
