@@ -117,6 +117,8 @@ int sxs_ensure_init(void)
 cudaStream_t sxs_default_stream(void) { return g_stream; }
 
 /* --------------------------------------------------------- expansion */
+#define EXPAND_POOL_MAX ((size_t)256 << 20)
+
 int sxsg_expand(const double *xyz, const double *vac, const double *dum, const double *sasa, double water_ff,
                 int natoms, const double *q, int Q, int L, double *spf_out)
 {
@@ -133,7 +135,9 @@ int sxsg_expand(const double *xyz, const double *vac, const double *dum, const d
 	for (int i = 0; i < natoms; i++) wf[i] = sasa ? water_ff * sasa[i] : 0.0;
 	/* one stream-ordered block for the call: the pool keeps it for the next
 	 * one, where nine device allocations and releases each synchronised
-	 * (1.0 of 2.8 ms at 3,500 atoms, L = 20, Q = 101) */
+	 * (1.0 of 2.8 ms at 3,500 atoms, L = 20, Q = 101).  A block above
+	 * EXPAND_POOL_MAX (16,000 atoms at L = 30) is the call's own and returned
+	 * at its end: there the allocation is small beside the kernels. */
 	size_t na = natoms > 0 ? (size_t)natoms : 1, off = 0, o[8];
 	const size_t bytes[8] = {sizeof(double) * 3 * na, sizeof(double) * na, sizeof(double) * na, sizeof(double) * na,
 	                         sizeof(double) * Q, sxsk_expand_ws_rad((int)na), sxsk_expand_ws_ylm((int)na, L),
@@ -143,7 +147,8 @@ int sxsg_expand(const double *xyz, const double *vac, const double *dum, const d
 		off += (bytes[i] + 255) / 256 * 256;
 	}
 	char *ws = NULL;
-	cudaError_t e = cudaMallocAsync((void **)&ws, off, s);
+	int pooled = off <= EXPAND_POOL_MAX;
+	cudaError_t e = pooled ? cudaMallocAsync((void **)&ws, off, s) : cudaMalloc((void **)&ws, off);
 	double *d_xyz = (double *)(ws + o[0]), *d_vac = (double *)(ws + o[1]), *d_dum = (double *)(ws + o[2]);
 	double *d_wf = (double *)(ws + o[3]), *d_q = (double *)(ws + o[4]), *d_rad = (double *)(ws + o[5]);
 	double2 *d_ylm = (double2 *)(ws + o[6]);
@@ -160,8 +165,9 @@ int sxsg_expand(const double *xyz, const double *vac, const double *dum, const d
 		sxs_count_launches(natoms > 0 ? sxsk_expand_launches() : 0);
 	}
 	if (!e) e = cudaMemcpyAsync(spf_out, d_out, sizeof(double) * spf_n, cudaMemcpyDeviceToHost, s);
-	if (ws) cudaFreeAsync(ws, s);
+	if (ws && pooled) cudaFreeAsync(ws, s);
 	if (!e) e = cudaStreamSynchronize(s);
+	if (ws && !pooled) cudaFree(ws);
 	free(wf);
 	if (e) return sxs_cuda_fail(e, "sxsg_expand");
 	return 0;
