@@ -679,8 +679,7 @@ static int capture(sxsg_batch *b, const blaunch *ls, int nl, int *ctr, const cha
 	for (int k = 0; k < 2 && !e; k++) e = cudaStreamWaitEvent(b->br[k], b->fork, 0);
 	for (int i = 0; i < b->n && !e && !rc; i++) {
 		if (b->v[i].nzt <= 0) continue;
-		rc = sxs_plan_ztables_on(b->plans[i], b->br[i & 1]);
-		nk += 3;
+		rc = sxs_plan_ztables_on(b->plans[i], b->br[i & 1], &nk);
 	}
 	int li = 0;
 	while (li < nl && ls[li].kind == 0 && !e && !rc) {

@@ -690,17 +690,18 @@ int sxsg_plan_set_poses(sxsg_plan *p, const int64_t *index, int64_t n, int skip)
 }
 
 /* per-z tables: Bessel values and translation matrices, computed in FP64 and
- * written in the form that the run's translation reads */
-static int plan_ztables(sxsg_plan *p, cudaStream_t s)
+ * written in the form that the run's translation reads; *nk += the kernels
+ * launched */
+static int plan_ztables(sxsg_plan *p, cudaStream_t s, int *nk)
 {
 	int L = p->L, Q = p->Q, form = p->fp32 ? SXSK_TAU_FP32 : (p->run_fixed ? SXSK_TAU_FIXED : SXSK_TAU_FP64);
 	SXS_K(sxsk_bessel_z(p->d_zt, p->nzt, p->d_q, Q, L, p->d_bes, s));
 	if (form == SXSK_TAU_FIXED) {
 		SXS_K(sxsk_fix_nu(p->d_bes, p->nzt, Q, L, p->d_nu2, s));
-		sxs_count_launches(1);
+		++*nk;
 	}
 	SXS_K(sxsk_tmatrix(p->d_bes, p->lt->d_dsymb, p->nzt, Q, L, p->lt->d_ll1, p->lt->nll1, p->d_nu2, p->d_tau, form, s));
-	sxs_count_launches(2);
+	*nk += 2;
 	return 0;
 }
 
@@ -713,15 +714,17 @@ static int plan_rotations(sxsg_plan *p);
 static int plan_tables(sxsg_plan *p)
 {
 	cudaStream_t s = p->s;
-	int side = p->nzt > 0 && p->s2, rc = 0;
+	int side = p->nzt > 0 && p->s2, rc = 0, nk = 0;
 	if (!side) {
 		rc = plan_rotations(p);
-		if (!rc && p->nzt > 0) rc = plan_ztables(p, s);
+		if (!rc && p->nzt > 0) rc = plan_ztables(p, s, &nk);
+		sxs_count_launches(nk);
 		return rc;
 	}
 	SXS_CU(cudaEventRecord(p->ev[2], s));
 	SXS_CU(cudaStreamWaitEvent(p->s2, p->ev[2], 0));
-	rc = plan_ztables(p, p->s2);
+	rc = plan_ztables(p, p->s2, &nk);
+	sxs_count_launches(nk);
 	cudaError_t e = cudaEventRecord(p->ev[3], p->s2);
 	if (!rc && !e) rc = plan_rotations(p);
 	if (!e) e = cudaStreamWaitEvent(s, p->ev[3], 0);
@@ -828,9 +831,9 @@ int sxs_plan_batch_view(sxsg_plan *p, sxs_plan_view *v)
 	return 0;
 }
 
-int sxs_plan_ztables_on(sxsg_plan *p, cudaStream_t s)
+int sxs_plan_ztables_on(sxsg_plan *p, cudaStream_t s, int *nk)
 {
-	return p->nzt > 0 ? plan_ztables(p, s) : 0;
+	return p->nzt > 0 ? plan_ztables(p, s, nk) : 0;
 }
 
 void sxs_plan_mark_run(sxsg_plan *p, int fit_mode, const float *ms)

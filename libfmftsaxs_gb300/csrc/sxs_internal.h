@@ -110,8 +110,9 @@ int sxs_plan_uses_fused(const sxsg_plan *p);
 /* fills v after uploading the twiddles of the plan's pose list (waits for
  * the plan's stream) */
 int sxs_plan_batch_view(sxsg_plan *p, sxs_plan_view *v);
-/* the per-z tables of the plan's touched z on stream s */
-int sxs_plan_ztables_on(sxsg_plan *p, cudaStream_t s);
+/* the per-z tables of the plan's touched z on stream s; *nk += the kernels
+ * launched */
+int sxs_plan_ztables_on(sxsg_plan *p, cudaStream_t s, int *nk);
 /* a batch filled the plan's outputs with this fit */
 void sxs_plan_mark_run(sxsg_plan *p, int fit_mode, const float *ms);
 
