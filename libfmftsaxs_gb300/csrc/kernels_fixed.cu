@@ -40,10 +40,14 @@ __device__ __forceinline__ int psym(int m, int K) { return m * K - m * (m - 1) /
 
 typedef long long i64;
 
+/* a b + c: a product and a sum, which the assembler joins to one IMAD.WIDE; the
+ * single instruction mad.wide.s32 comes out with a second one beside it (16
+ * independent sums: 7.6 against 8.5 T/s, 2.1 instructions per product), and
+ * as a C expression the sums are reordered and not joined */
 __device__ __forceinline__ i64 madw(int a, int b, i64 c)
 {
 	i64 r;
-	asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+	asm("{\n\t.reg .s64 t;\n\tmul.wide.s32 t, %1, %2;\n\tadd.s64 %0, t, %3;\n\t}" : "=l"(r) : "r"(a), "r"(b), "l"(c));
 	return r;
 }
 
@@ -226,9 +230,10 @@ __device__ __forceinline__ FixTw fix_tw(const double2 *tw, int k, int N)
  * y(m1) - y(-m1) (12 IMAD.WIDE and ~40 adds and shifts) and per gamma pair
  * four sums of 16 IMAD.WIDE in all, ~75 clocks of its pipe, where the FP64
  * form's 8 operations take 512.  Bound by that pipe; table stage (both tables,
- * per-z tables beside) at L = 20, Q = 101: 17.0 -> 4.0 ms. */
+ * per-z tables beside) at L = 20, Q = 101: 17.0 -> 3.5 ms (six gamma pairs: four
+ * blocks on an SM, 166 registers instead of 178 and 4.3 ms). */
 template <int G>
-__global__ void __launch_bounds__(FROT_THREADS)
+__global__ void __launch_bounds__(FROT_THREADS, (G == 6 ? 4 : 0))
 k_fix_rotate(const int4 *__restrict__ spf, const int2 *__restrict__ dtab, const double2 *__restrict__ tw, int Q, int L,
              int4 *__restrict__ out)
 {
@@ -323,8 +328,8 @@ k_fix_rotate(const int4 *__restrict__ spf, const int2 *__restrict__ dtab, const 
  * registers; block = (tile, half a slice of combos sharing z, m), tau^m(q z)
  * staged in shared memory.  Rows in even/odd pairs, so that the parity of i +
  * k, which says whether an entry adds tau U or tau (-i U), is known at compile
- * time.  Bound by IMAD.WIDE: 6 per (i, k), 14.3 of the 16.0 ms at L = 20, Q =
- * 101, 70,000 poses (FP64: 59); 8 combos per block instead of the FP64
+ * time.  Bound by IMAD.WIDE: 6 per (i, k); 15.0 ms at L = 20, Q = 101, 70,000
+ * poses (FP64: 59); 8 combos per block instead of the FP64
  * form's 16 so that two to four blocks' staging overlaps. */
 template <int PAR, int NB>
 __device__ __forceinline__ int4 fix_row(const int2 *__restrict__ row, const int4 (&u)[NB])
@@ -451,12 +456,12 @@ __device__ __forceinline__ i64 join(i64 x, i64 y, int d)
  * two of a pair (P_a R_b and P_b R_a, whose units differ) joined in the larger
  * unit, and the pose's phase w_m is applied to the six sums.  Bound by
  * the integer pipe: 108 IMAD.WIDE per pair of rows.  At L = 20, Q = 101,
- * 70,000 poses: 25.1 ms (FP64 kernel: 87.5).  With one unit for all channels
- * six products do, (P_a + P_b)(R_a + R_b) - P_a R_a - P_b R_b, in 18.9 ms, but
- * a channel ten times weaker then has up to 7 times the FP64 kernels' error
- * (a thousand times: 500); the same six with one operand of each sum shifted to
- * the other's unit 26.1; a thread per channel of P 26.9; Im P negated once
- * instead of Im R 25.1 against 25.7; two blocks per SM 28.7. */
+ * 70,000 poses: 22.9 ms (FP64 kernel: 87.5).  With one unit for all channels
+ * six products do, (P_a + P_b)(R_a + R_b) - P_a R_a - P_b R_b, but a channel ten
+ * times weaker then has up to 7 times the FP64 kernels' error (a thousand times:
+ * 500); the same six with one operand of each sum shifted to the other's unit
+ * 28.7; a thread per channel of P 23.7; rows two pairs ahead 23.8; mad.wide.s32
+ * 25.1. */
 __global__ void __launch_bounds__(FPC_THREADS, 3)
 k_fix_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int ncombo,
             const int32_t *__restrict__ combo_zbg, const int4 *__restrict__ P, const int4 *__restrict__ R,
