@@ -188,19 +188,27 @@ class Clocks:
 # DRAM bytes per pose of the dominant kernel from ncu captures of the same
 # kernel on the poses of this workload with translation z index < 3 (the
 # same poses per translated row as the whole list, profiles/): the traffic
-# of a launch scales with the poses it processes at that density.  The FP64
-# figure is of the floating-point kernel; the fixed-point one reads rows of
-# the same size.
-TRAFFIC_PER_POSE = {("c1", "mixed"): 9.13e4, ("c1", "fp64"): 4.47e5}
+# of a launch scales with the poses it processes at that density.  FP64: the
+# fixed-point kernel, z index < 1.
+TRAFFIC_PER_POSE = {("c1", "mixed"): 9.13e4, ("c1", "fp64"): 4.19e5}
+# 32 x 32 + 64-bit integer multiply-adds per clock and SM (register-resident
+# chains, measured), of 152 SMs: the unit of the plain path's fixed-point
+# kernels (L <= 31)
+IMAD_PER_CLOCK, SMS = 28, 152
 # L2-to-SM bytes per pose of the FP32 per-pose kernel (ncu
 # l1tex__m_xbar2l1tex_read_sectors on the same capture): the P row of every
 # pose (no block shares one) and the R rows, which the poses of a warp share.
 L2_TO_SM_PER_POSE = {("c1", "mixed"): 6.18e5}
 
 
-def pose_flops(L, Q, precision):
-    """Algorithmic FLOPs of the per-pose contraction for one pose (the same
-    count for both precisions): over the (L+1)(L+2)/2 pairs
+def pose_imads(L, Q):
+    """Integer multiply-adds of the fixed-point per-pose kernel for one pose: 9
+    complex products of 4 real ones, 3 each, per pair (m >= 0, l >= m) and q."""
+    return Q * ((L + 1) * (L + 2) // 2) * 108
+
+
+def pose_flops(L, Q):
+    """Algorithmic FLOPs of the per-pose contraction for one pose: over the (L+1)(L+2)/2 pairs
     (m >= 0, l >= m) and Q q values, the phase w_m applied to the 3 channels
     of R (3 complex multiplies, 18 FLOPs) and the real parts of the 9
     channel products (36 FLOPs)."""
@@ -303,12 +311,11 @@ def accuracy(mix, ref, k=100, topk=None):
     return out
 
 
-def expansion_timing(g, w, fp64_peak):
+def expansion_timing(g, w):
     """The A_lm expansion per molecule (sxsg_expand, with its transfers of a
     few MB) and its rate over the accumulation's 12 FLOPs per atom, q and
-    (l, m) (3 channels of complex-by-real multiply-adds), as equivalent FP64
-    operations: the accumulation itself runs in fixed point on the integer
-    multiply-add pipe, so the fraction of the FP64 pipe's peak may pass 1."""
+    (l, m) (3 channels of complex-by-real multiply-adds), which runs in fixed
+    point on the integer pipe beside the series on the FP64 pipe."""
     out = {}
     water = g.ff_water()
     for name, m in (("receptor", w.rec), ("ligand", w.lig)):
@@ -322,8 +329,7 @@ def expansion_timing(g, w, fp64_peak):
             ts.append(g.timer_stop())
         ms = float(np.median(ts))
         tf = 12.0 * m.natoms * w.Q * (w.L + 1) ** 2 / (ms * 1e-3) / 1e12
-        out[name] = {"atoms": m.natoms, "ms": ms, "fp64_tflops": tf,
-                     "fp64_frac": tf / fp64_peak if fp64_peak > 0 else None}
+        out[name] = {"atoms": m.natoms, "ms": ms, "accumulation_tflops": tf}
     return out
 
 
@@ -638,9 +644,11 @@ def run_ours(args):
     h2d = w.A.nbytes + w.B.nbytes + w.q.nbytes + w.z.nbytes + w.a.nbytes + idx.nbytes + w.c1g.nbytes + w.c2g.nbytes
     d2h = 3 * 8 * n
 
-    pf = pose_flops(w.L, w.Q, head) * n
-    achieved = pf / (stage[2] * 1e-3) / 1e12
+    fixed = head == "fp64" and w.L <= 31
+    achieved = (pose_imads(w.L, w.Q) if fixed else pose_flops(w.L, w.Q)) * n / (stage[2] * 1e-3) / 1e12
     peak = fp32_peak if head == "mixed" else fp64_peak
+    if fixed:
+        peak = IMAD_PER_CLOCK * SMS * ((clocks or {}).get("sm_mhz") or 0.0) * 1e-6
     fref = reference_flops(w)
     tkey = (args.config, head)
     traffic = TRAFFIC_PER_POSE[tkey] * n / nchunks if tkey in TRAFFIC_PER_POSE else None
@@ -668,19 +676,19 @@ def run_ours(args):
                  "stages_ms": dict(zip(("tables", "translate", "pose", "fit"), runs["fp64"][1][:4].tolist()))},
         "reference_flops_per_step": fref,
         "reference_equiv_tflops": fref / (ms * 1e-3) / 1e12,
-        "roofline": {"bound": "fp32" if head == "mixed" else "fp64",
-                     "kernel": "k_pose_cross<float>" if head == "mixed" else "k_fix_cross",
-                     "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+        "roofline": {"bound": "fp32" if head == "mixed" else ("imad" if fixed else "fp64"),
+                     "kernel": "k_fix_cross" if fixed else "k_pose_cross<%s>" % ("float" if head == "mixed" else "double"),
+                     "achieved": achieved, "peak": peak, "unit": "T multiply-adds/s" if fixed else "TFLOP/s",
                      "frac": achieved / peak if peak > 0 else None,
                      "traffic": traffic,
                      "traffic_source": "ncu DRAM read+write per pose of the same kernel on the poses with z index < 3 "
                                        "(z index < 1 for FP64), "
                                        "scaled to the poses of one launch (%d chunk(s) per run)" % nchunks,
                      "hbm_frac": (traffic * nchunks / (stage[2] * 1e-3) / 1e9 / 6773.5) if traffic else None,
-                     "peak_source": "measured in this run: register-resident FP32 FMA chains on every SM"
-                                    if head == "mixed" else
-                                    "measured in this run: register-resident FP64 FMA chains on every SM (the kernel "
-                                    "does the equivalent operations in fixed point on the integer pipe)"},
+                     "peak_source": "%d 32 x 32 + 64-bit integer multiply-adds per clock and SM (measured) at this run's "
+                                    "SM clock" % IMAD_PER_CLOCK if fixed else
+                                    "measured in this run: register-resident %s FMA chains on every SM"
+                                    % ("FP32" if head == "mixed" else "FP64")},
         "cpu_baseline": cpu_baseline_entry(w, cs, kind) if cs else None,
         "e2e": {"value": n / e2e_s, "unit": "poses/s", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": int(launches),
@@ -710,7 +718,7 @@ def run_ours(args):
                 p.close()
         out["accuracy"] = accuracy(res, runs["fp64"][3], topk=tk)
         out["accuracy"].update(iq_accuracy(g, w))
-    out["expansion"] = expansion_timing(g, w, fp64_peak)
+    out["expansion"] = expansion_timing(g, w)
     if not args.skip_serve:
         out["serving"] = run_serving(g, args)
     if not args.skip_batch:
