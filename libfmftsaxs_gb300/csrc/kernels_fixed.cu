@@ -429,13 +429,24 @@ __device__ __forceinline__ int4 ld_pol(const int4 *p, uint64_t pol)
 	return v;
 }
 
-/* (re, im) += p r for complex limbs, n = -Im p */
-__device__ __forceinline__ void cmul_add(Acc &re, Acc &im, int4 p, int2 n, int4 r)
+/* the real and the imaginary part of p r for complex limbs, n = -Im p */
+__device__ __forceinline__ void re_add(Acc &s, int4 p, int2 n, int4 r)
 {
-	mul_add(re, p.x, p.y, r.x, r.y);
-	mul_add(re, n.x, n.y, r.z, r.w);
-	mul_add(im, p.x, p.y, r.z, r.w);
-	mul_add(im, p.z, p.w, r.x, r.y);
+	s.hh = madw(p.x, r.x, s.hh);
+	s.mid = madw(p.x, r.y, s.mid);
+	s.hh = madw(n.x, r.z, s.hh);
+	s.mid = madw(p.y, r.x, s.mid);
+	s.mid = madw(n.x, r.w, s.mid);
+	s.mid = madw(n.y, r.z, s.mid);
+}
+__device__ __forceinline__ void im_add(Acc &s, int4 p, int4 r)
+{
+	s.hh = madw(p.x, r.z, s.hh);
+	s.mid = madw(p.x, r.w, s.mid);
+	s.hh = madw(p.z, r.x, s.hh);
+	s.mid = madw(p.y, r.z, s.mid);
+	s.mid = madw(p.z, r.y, s.mid);
+	s.mid = madw(p.w, r.x, s.mid);
 }
 
 #define FPC_POSES 16
@@ -455,8 +466,8 @@ __device__ __forceinline__ i64 join(i64 x, i64 y, int d)
  * Per m the nine channel products are summed over l as complex numbers, the
  * two of a pair (P_a R_b and P_b R_a, whose units differ) joined in the larger
  * unit, and the pose's phase w_m is applied to the six sums.  Bound by
- * the integer pipe: 108 IMAD.WIDE per pair of rows.  At L = 20, Q = 101,
- * 70,000 poses: 22.9 ms (FP64 kernel: 87.5).  With one unit for all channels
+ * the integer pipe: 108 IMAD.WIDE per pair of rows, 54 at m = 0.  At L = 20, Q =
+ * 101, 70,000 poses: 21.5 ms (FP64 kernel: 87.5; all 108 at m = 0: 22.8).  With one unit for all channels
  * six products do, (P_a + P_b)(R_a + R_b) - P_a R_a - P_b R_b, but a channel ten
  * times weaker then has up to 7 times the FP64 kernels' error (a thousand times:
  * 500); the same six with one operand of each sum shifted to the other's unit
@@ -519,15 +530,26 @@ k_fix_cross(const sxsk_pose *__restrict__ poses, int npose, int combo_base, int 
 			r1 = ld_pol(Rr + SXS_QT, polR);
 			r2 = ld_pol(Rr + 2 * SXS_QT, polR);
 			int2 n0 = make_int2(-a0.z, -a0.w), n1 = make_int2(-a1.z, -a1.w), n2 = make_int2(-a2.z, -a2.w);
-			cmul_add(re[0], im[0], a0, n0, b0);
-			cmul_add(re[1], im[1], a0, n0, b1);
-			cmul_add(re[2], im[2], a0, n0, b2);
-			cmul_add(re[3], im[3], a1, n1, b1);
-			cmul_add(re[4], im[4], a1, n1, b2);
-			cmul_add(re[5], im[5], a2, n2, b2);
-			cmul_add(re[6], im[6], a1, n1, b0);
-			cmul_add(re[7], im[7], a2, n2, b0);
-			cmul_add(re[8], im[8], a2, n2, b1);
+			re_add(re[0], a0, n0, b0);
+			re_add(re[1], a0, n0, b1);
+			re_add(re[2], a0, n0, b2);
+			re_add(re[3], a1, n1, b1);
+			re_add(re[4], a1, n1, b2);
+			re_add(re[5], a2, n2, b2);
+			re_add(re[6], a1, n1, b0);
+			re_add(re[7], a2, n2, b0);
+			re_add(re[8], a2, n2, b1);
+			if (m > 0) {   /* w_0 = 1: only real parts count */
+				im_add(im[0], a0, b0);
+				im_add(im[1], a0, b1);
+				im_add(im[2], a0, b2);
+				im_add(im[3], a1, b1);
+				im_add(im[4], a1, b2);
+				im_add(im[5], a2, b2);
+				im_add(im[6], a1, b0);
+				im_add(im[7], a2, b0);
+				im_add(im[8], a2, b1);
+			}
 		}
 		/* F += Re(w_m G): the sums start with m = 0, which counts once where
 		 * the others count twice (their mirror images) */

@@ -847,7 +847,7 @@ void sxs_plan_mark_run(sxsg_plan *p, int fit_mode, const float *ms)
 /* The contraction tables of a run.  On the plain path the fixed-point kernels
  * (kernels_fixed.cu) take a quarter of the FP64 ones' time (L = 20, Q = 101,
  * 70,000 poses: tables 3.5 against 17.0 ms, translation 15.0 / 59.2, poses
- * 22.9 / 87.5) and are as close to the exact sums, each channel pair by its own
+ * 21.5 / 87.5) and are as close to the exact sums, each channel pair by its own
  * norms; they hold a column in registers up to L = 31.  The L-BFGS-B fit keeps
  * the FP64 kernels: its stopping point moves by up to 1e-6 in (c1, c2) when the
  * last bits of its input change. */
