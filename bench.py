@@ -190,7 +190,7 @@ class Clocks:
 # same poses per translated row as the whole list, profiles/): the traffic
 # of a launch scales with the poses it processes at that density.  FP64: the
 # fixed-point kernel, z index < 1.
-TRAFFIC_PER_POSE = {("c1", "mixed"): 9.13e4, ("c1", "fp64"): 4.19e5}
+TRAFFIC_PER_POSE = {("c1", "mixed"): 9.13e4, ("c1", "fp64"): 4.25e5}
 # 32 x 32 + 64-bit integer multiply-adds per clock and SM (register-resident
 # chains, measured), of 152 SMs: the unit of the plain path's fixed-point
 # kernels (L <= 31)
@@ -203,8 +203,9 @@ L2_TO_SM_PER_POSE = {("c1", "mixed"): 6.18e5}
 
 def pose_imads(L, Q):
     """Integer multiply-adds of the fixed-point per-pose kernel for one pose: 9
-    complex products of 4 real ones, 3 each, per pair (m >= 0, l >= m) and q."""
-    return Q * ((L + 1) * (L + 2) // 2) * 108
+    complex products of 4 real ones (2 at m = 0), 3 each, per pair (m >= 0, l >=
+    m) and q."""
+    return Q * (L + 1) * (108 * (L + 2) // 2 - 54)
 
 
 def pose_flops(L, Q):
