@@ -356,15 +356,16 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c)
  * weights w_ch, scaled by the largest exponent in the chunk to 53-bit
  * integers h 2^27 + l, times the limbs of Y (h 2^27 + l, 54 bits) as three
  * 32 x 32 + 64-bit multiply-adds (h h', and h l' + l h'), sums exact; a
- * chunk's sums are added to the thread's in double.  Bound by the FP64 pipe:
+ * chunk's sums are added to the thread's in double.  A coefficient is accurate
+ * relative to sum |f j_l| times the bound of |Y_lm|, not to its own size where
+ * all Y_lm are small (large m, atoms near the z axis).  Bound by the FP64 pipe:
  * 2 operations per series term (8.4 terms on average, the longest of each
  * warp) and ~16 more per (atom, q, l), beside 18 IMAD.WIDE (~83 clocks) per
  * (atom, l, m); the FP64 form had 9 per term and 6 per (atom, l, m).  The
- * whole call (with k_ylm and one stream-ordered work buffer) 3,500 atoms, L =
- * 20, Q = 101: 4.9 -> 1.4 ms; 8,000, L = 30, Q = 201: 36.2 -> 9.9.
- * Blocks per SM (10: 48 registers, some spilled outside the loops): whole
- * call 1.54 / 11.1 ms with 7, 1.39 / 9.9 with 9, 1.31 / 8.9 with 10, 1.72 /
- * 11.8 with 11. */
+ * whole call (with k_ylm and one work buffer) 3,500 atoms, L = 20, Q = 101: 4.9
+ * -> 1.44 ms; 8,000, L = 30, Q = 201: 36.2 -> 9.92.  Blocks per SM (10: 48
+ * registers, some spilled outside the loops): 1.45 / 10.4 ms with 8, 1.41 /
+ * 9.99 with 9. */
 __global__ void __launch_bounds__(EXP_THREADS, 10) k_expand_fix(const int4 *__restrict__ ylm,
                                                              const double *__restrict__ rad,
                                                              const double *__restrict__ vac,
@@ -492,26 +493,6 @@ __device__ __forceinline__ void tau_store(double *o, double v, double) { *o = v;
 __device__ __forceinline__ void tau_store(float *o, double v, double) { *o = (float)v; }
 __device__ __forceinline__ void tau_store(int2 *o, double v, double c28) { *o = sxs_limbs(v, c28); }
 
-/* T^{|m|}_{l l1}(q z) = sum_p (-1)^m i^p j_p d_lm(l1,p) for l <= l1, mirrored
- * (src/fftsaxs.c:182-243).  Thread = (iz, m, (m <= l, l1 >= l), q), q fastest;
- * nbx blocks per (iz, m), those past its pairs return at once.
- * Output in the q-tiled layout of the contraction tables (tiles of SXS_QT q,
- * zeros past Q), entries with l, l1 >= m only (no others are read).
- * The 3j factor 3j(l p l1; 0 0 0) vanishes unless l + p + l1 is even, so T
- * is real for even l + l1 and imaginary for odd l + l1 (the other part is
- * the sum of exact zeros and binary128 round-off below 1e-30 relative); the
- * table keeps that one real number, tau = Re T (even) or Im T (odd), in the
- * form that the run's translation reads.
- * The reference sums Re and Im with i^p in {1, i, -1, -i}; for the component
- * kept here the terms with p of the other parity add +-0, so summing only p
- * = l + l1 (mod 2), in the same order, gives the same value bit for bit; the
- * signs of (-1)^m and i^p are exact and turn the sum into alternate sums and
- * differences of the products: two FP64 operations per term (four with the
- * signs multiplied in), 63 % of that pipe's rate at L = 30; one, where the
- * sum is not stored as a double (tm_value).  With the float
- * form written here, not by a pass over a double table, 16 z of the mixed
- * path take 0.25 + 0.04 -> 0.20 ms at L = 20, Q = 101 and 2.14 + 0.29 -> 1.69
- * ms at L = 30, Q = 201. */
 /* sum over p = p0, p0 + 2, ..., p1 of +- dp[p] bp[p Q], the sign alternating
  * from neg: products and sums rounded one by one */
 __device__ __forceinline__ double tm_sum(const double *dp, const double *bp, int Q, int p0, int p1, bool neg)
@@ -562,6 +543,25 @@ __device__ __forceinline__ double tm_value(float *, const double *dp, const doub
 	return (float)(v - d) == (float)(v + d) ? v : tm_sum(dp, bp, Q, p0, p1, neg);
 }
 
+/* T^{|m|}_{l l1}(q z) = sum_p (-1)^m i^p j_p d_lm(l1,p) for l <= l1, mirrored
+ * (src/fftsaxs.c:182-243).  Thread = (iz, m, (m <= l, l1 >= l), q), q fastest;
+ * nbx blocks per (iz, m), those past its pairs return at once.
+ * Output in the q-tiled layout of the contraction tables (tiles of SXS_QT q,
+ * zeros past Q), entries with l, l1 >= m only (no others are read).
+ * The 3j factor 3j(l p l1; 0 0 0) vanishes unless l + p + l1 is even, so T
+ * is real for even l + l1 and imaginary for odd l + l1 (the other part is
+ * the sum of exact zeros and binary128 round-off below 1e-30 relative); the
+ * table keeps that one real number, tau = Re T (even) or Im T (odd), in the
+ * form that the run's translation reads.
+ * The reference sums Re and Im with i^p in {1, i, -1, -i}; for the component
+ * kept here the terms with p of the other parity add +-0, so summing only p
+ * = l + l1 (mod 2), in the same order, gives the same value bit for bit; the
+ * signs of (-1)^m and i^p are exact and turn the sum into alternate sums and
+ * differences of the products: two FP64 operations per term (four with the
+ * signs multiplied in), one where the sum is not stored as a double (tm_value).
+ * Bound by that pipe (89 % busy).  16 z of the mixed path, with the float form
+ * written here and not by a pass over a double table: 0.29 -> 0.14 ms at L =
+ * 20, Q = 101, 2.43 -> 0.78 at L = 30, Q = 201. */
 template <typename T>
 __global__ void __launch_bounds__(128) k_tmatrix(const double *__restrict__ bes, const double *__restrict__ ds, int nz,
                                                  int Q, int L, const int2 *__restrict__ ll1, int nll1, int nbx,

@@ -5,7 +5,7 @@
  *
  * This GPU's FP64 pipe takes 2 multiply-adds per clock and SM (measured 0.50
  * T/s over the GPU); its 32 x 32 + 64-bit integer multiply-add (IMAD.WIDE)
- * takes 28 (4.6 clocks per warp and scheduler).  A real number v of a table
+ * takes 27 (8.5 T/s).  A real number v of a table
  * row is held as v / 2^e = (h 2^29 + l) 2^-57 with two 32-bit limbs, |l| <=
  * 2^28, and one exponent e per molecule, channel and q; a product is then
  * three IMAD.WIDE,
