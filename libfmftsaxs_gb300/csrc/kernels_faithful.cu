@@ -363,10 +363,13 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c)
  * warp) and ~16 more per (atom, q, l), beside 18 IMAD.WIDE (~83 clocks) per
  * (atom, l, m); the FP64 form had 9 per term and 6 per (atom, l, m).  The
  * whole call (with k_ylm and one work buffer) 3,500 atoms, L = 20, Q = 101: 4.9
- * -> 1.44 ms; 8,000, L = 30, Q = 201: 36.2 -> 9.92.  Blocks per SM (10: 48
- * registers, some spilled outside the loops): 1.45 / 10.4 ms with 8, 1.41 /
- * 9.99 with 9. */
-__global__ void __launch_bounds__(EXP_THREADS, 10) k_expand_fix(const int4 *__restrict__ ylm,
+ * -> 1.43 ms; 8,000, L = 30, Q = 201: 36.2 -> 9.93; 4,909, L = 16, Q = 124:
+ * 1.94.  NB, blocks per SM: 9 (56 registers) or, from L = EXP_NB10 on, 10 (48, more
+ * spilled): 1.43 / 9.93 / 1.94 ms for these three with 9, 1.44 / 9.86 / 2.03 with
+ * 10, 1.45 / 10.4 for the first two with 8. */
+#define EXP_NB10 24
+template <int NB>
+__global__ void __launch_bounds__(EXP_THREADS, NB) k_expand_fix(const int4 *__restrict__ ylm,
                                                              const double *__restrict__ rad,
                                                              const double *__restrict__ vac,
                                                              const double *__restrict__ dum,
@@ -760,7 +763,8 @@ int sxsk_expand(const double *xyz, const double *vac, const double *dum, const d
 	size_t qsm = sizeof(double2) * (size_t)K * L / 2;   /* at most 29 KB (L = 60) */
 	if (fixed) {
 		k_ylm<int4, true><<<nblk(natoms, YLM_ATOMS), YLM_THREADS, qsm, s>>>(xyz, natoms, L, ynorm, (int4 *)ylm_ws, rad_ws);
-		k_expand_fix<<<Q * K, EXP_THREADS, 0, s>>>((const int4 *)ylm_ws, rad_ws, vac, dum, wfac, natoms, q, Q, L, spf_out);
+		auto kern = L < EXP_NB10 ? k_expand_fix<9> : k_expand_fix<10>;
+		kern<<<Q * K, EXP_THREADS, 0, s>>>((const int4 *)ylm_ws, rad_ws, vac, dum, wfac, natoms, q, Q, L, spf_out);
 	} else {
 		k_ylm<double2, false><<<nblk(natoms, YLM_ATOMS), YLM_THREADS, qsm, s>>>(xyz, natoms, L, ynorm, ylm_ws, rad_ws);
 		k_expand_ql<<<Q * K, EXP_THREADS, 0, s>>>(ylm_ws, rad_ws, vac, dum, wfac, natoms, q, Q, L, spf_out);
